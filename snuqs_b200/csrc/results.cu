@@ -14,10 +14,10 @@
 // amplitudes, then pairs of pairs, ...), and a shot with uniform u walks that
 // tree from the root with r = u * total: at a node with children sums (L, R)
 // it goes left when r < L or R == 0, else subtracts L and goes right.  The
-// tree is split at leaves of 2^12 amplitudes: the levels above the leaves
-// stay in device memory, the levels inside a leaf are rebuilt in shared
-// memory by the block that serves the leaf's shots.  Any restatement that
-// sums in the same tree and walks it the same way returns the same indices.
+// tree is cut at nodes of 2^7 amplitudes: the levels from there up stay in
+// device memory, the levels inside a node are rebuilt in registers by the warp
+// that serves a shot.  Any restatement that sums in the same tree and walks
+// it the same way returns the same indices.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -35,183 +35,217 @@
 
 namespace {
 
-constexpr int kLeafBits = 12;
-constexpr uint32_t kLeafAmps = 1u << kLeafBits;
-constexpr int kLeafThreads = 256;
-constexpr uint32_t kPerThread = kLeafAmps / kLeafThreads;  // 16 consecutive amplitudes
+// Amplitudes of one block of the first pass, and the size of the nodes that
+// the stored tree ends at: 2^7 amplitudes up to 30 qubits, then as large as
+// keeps the stored tree at 2^24 doubles (128 MiB).
+constexpr int kBlockBits = 12;
+constexpr uint32_t kBlockAmps = 1u << kBlockBits;
+constexpr int kTreeThreads = 256;
+constexpr uint32_t kPerLane = kBlockAmps / kTreeThreads;  // 16 amplitudes, 32 apart
+constexpr uint32_t kNodeBits = 7;
+constexpr uint32_t kMaxTreeDepth = 23;
+
+uint32_t node_bits(uint32_t n) { return n > kNodeBits + kMaxTreeDepth ? n - kMaxTreeDepth : kNodeBits; }
 
 template <typename C2>
-__device__ __forceinline__ double prob(const C2 *__restrict__ psi, uint64_t i, uint64_t N) {
-  if (i >= N) return 0.0;  // states below 2^12 amplitudes are padded with zeros
-  const C2 a = psi[i];
+__device__ __forceinline__ double prob_of(const C2 &a) {
   const double re = double(a.x), im = double(a.y);
   return __dadd_rn(__dmul_rn(re, re), __dmul_rn(im, im));
 }
 
-// Sum of one leaf in the fixed tree (pairwise sums over consecutive
-// amplitudes, level by level).  Warp w covers the 512 amplitudes from
-// 512 w; lane l reads amplitude 32 k + l for k = 0..15 (coalesced), the five
-// lowest levels of each group of 32 are lane pairs l, l^1, l^2, ... (shuffles;
-// a commutative add gives both partners the same value), the next four are
-// the groups k in registers, then the warps pairwise through shared memory.
+// First pass (bound: one read of the state): the sums of the fixed tree (pairs
+// of consecutive amplitudes, level by level) from nodes of 2^node_bits up to
+// 2^12 amplitudes.  Heap layout: the 2^d nodes of depth d at tree + 2^d, so the
+// root is tree[1] and the children of node k are the 16-byte pair 2k, 2k + 1.
+// Warp w covers the 512 amplitudes from 512 w; lane l reads amplitude 32 k + l
+// for k = 0..15 (coalesced), the five lowest levels of each group of 32 are
+// lane pairs l, l^1, l^2, ... (shuffles; a commutative add gives both partners
+// the same value), the next four are the groups k in registers, then the
+// warps pairwise through shared memory.
 template <typename C2>
-__global__ void __launch_bounds__(kLeafThreads) leaf_sum_kernel(const C2 *__restrict__ psi, uint64_t N,
-                                                                double *__restrict__ leaves) {
-  __shared__ double ws[kLeafThreads / 32];
-  const uint32_t lane = threadIdx.x & 31u;
-  const uint64_t base = uint64_t(blockIdx.x) * kLeafAmps + uint64_t(threadIdx.x >> 5) * (32 * kPerThread) + lane;
-  double v[kPerThread];
+__global__ void __launch_bounds__(kTreeThreads) node_sum_kernel(const C2 *__restrict__ psi, uint32_t n,
+                                                                uint32_t node, double *__restrict__ tree) {
+  __shared__ double ws[kTreeThreads / 32];
+  const uint64_t N = uint64_t(1) << n;
+  const int depth = n > node ? int(n - node) : 0;  // of the nodes of 2^node amplitudes
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  const uint64_t base = uint64_t(blockIdx.x) * kBlockAmps + uint64_t(warp) * (32 * kPerLane) + lane;
+  double v[kPerLane];
 #pragma unroll
-  for (uint32_t k = 0; k < kPerThread; ++k) v[k] = prob(psi, base + 32 * k, N);
+  for (uint32_t k = 0; k < kPerLane; ++k)  // states below 2^12 amplitudes are padded with zeros
+    v[k] = base + 32 * k < N ? prob_of(psi[base + 32 * k]) : 0.0;
+  // Node j of this block at the level of 2^s amplitudes.
+  auto put = [&](uint32_t s, uint32_t j, double x) {
+    const int d = depth - int(s - node);
+    if (d < 0) return;
+    const uint64_t at = uint64_t(blockIdx.x) * (kBlockAmps >> s) + j;
+    if (at < (uint64_t(1) << d)) tree[(uint64_t(1) << d) + at] = x;
+  };
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1)
 #pragma unroll
-    for (uint32_t k = 0; k < kPerThread; ++k) v[k] = __dadd_rn(v[k], __shfl_xor_sync(0xffffffffu, v[k], o));
+    for (uint32_t k = 0; k < kPerLane; ++k) v[k] = __dadd_rn(v[k], __shfl_xor_sync(0xffffffffu, v[k], o));
 #pragma unroll
-  for (uint32_t w = kPerThread / 2; w >= 1; w >>= 1)
+  for (uint32_t w = kPerLane / 2, s = 6; w >= 1; w >>= 1, ++s) {
 #pragma unroll
     for (uint32_t j = 0; j < w; ++j) v[j] = __dadd_rn(v[2 * j], v[2 * j + 1]);
-  const double s = v[0];
-  if (lane == 0) ws[threadIdx.x >> 5] = s;
+    if (s >= kNodeBits && s >= node && lane == 0) {
+#pragma unroll
+      for (uint32_t j = 0; j < w; ++j) put(s, warp * w + j, v[j]);
+    }
+  }
+  if (lane == 0) ws[warp] = v[0];
   __syncthreads();
   if (threadIdx.x == 0) {
-    double w[kLeafThreads / 32];
+    double w[kTreeThreads / 32];
 #pragma unroll
-    for (int j = 0; j < kLeafThreads / 32; ++j) w[j] = ws[j];
+    for (int j = 0; j < kTreeThreads / 32; ++j) w[j] = ws[j];
 #pragma unroll
-    for (int m = kLeafThreads / 64; m >= 1; m >>= 1)
+    for (uint32_t m = kTreeThreads / 64, s = 10; m >= 1; m >>= 1, ++s)
 #pragma unroll
-      for (int j = 0; j < m; ++j) w[j] = __dadd_rn(w[2 * j], w[2 * j + 1]);
-    leaves[blockIdx.x] = w[0];
+      for (uint32_t j = 0; j < m; ++j) {
+        w[j] = __dadd_rn(w[2 * j], w[2 * j + 1]);
+        if (s >= node) put(s, j, w[j]);
+      }
   }
 }
 
-// Levels above the leaves: level d (2^d nodes) at tree + 2^d - 1, so the root
-// is tree[0] and the leaves (depth D) start at tree + 2^D - 1.
-__global__ void __launch_bounds__(1024) upper_tree_kernel(double *__restrict__ tree, uint32_t depth) {
-  for (int d = int(depth) - 1; d >= 0; --d) {
-    const uint64_t nodes = uint64_t(1) << d;
-    double *lv = tree + (nodes - 1), *ch = tree + (2 * nodes - 1);
-    for (uint64_t k = threadIdx.x; k < nodes; k += blockDim.x) lv[k] = __dadd_rn(ch[2 * k], ch[2 * k + 1]);
+// `levels` (1..11) levels above depth `from`: block b sums the 2^levels nodes
+// from node b << levels, through shared memory.
+constexpr uint32_t kUpperLevels = 11;
+__global__ void __launch_bounds__(1024) upper_tree_kernel(double *__restrict__ tree, uint32_t from, uint32_t levels) {
+  __shared__ double buf[2][1u << (kUpperLevels - 1)];
+  uint32_t nodes = 1u << levels;
+  const double2 *src = reinterpret_cast<const double2 *>(tree + ((uint64_t(1) << from) + (uint64_t(blockIdx.x) << levels)));
+  for (uint32_t l = 1; l <= levels; ++l) {
+    nodes >>= 1;
+    const uint64_t at = (uint64_t(1) << (from - l)) + (uint64_t(blockIdx.x) << (levels - l));
+    if (threadIdx.x < nodes) {
+      const double2 c = l == 1 ? src[threadIdx.x] : reinterpret_cast<const double2 *>(buf[l & 1])[threadIdx.x];
+      const double x = __dadd_rn(c.x, c.y);
+      tree[at + threadIdx.x] = x;
+      buf[(l + 1) & 1][threadIdx.x] = x;
+    }
     __syncthreads();
   }
 }
 
 __device__ __forceinline__ bool go_left(double r, double l, double rr) { return r < l || rr == 0.0; }
 
-// Per shot: r = u * total, walk down to a leaf; count the shots per leaf.
-__global__ void shot_descend_kernel(const double *__restrict__ tree, uint32_t depth,
-                                    const double *__restrict__ u, uint64_t shots, uint32_t *__restrict__ leaf,
-                                    double *__restrict__ resid, uint32_t *__restrict__ count) {
-  const uint64_t s = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (s >= shots) return;
-  double r = __dmul_rn(u[s], tree[0]);
-  uint64_t k = 0;
-  for (uint32_t d = 0; d < depth; ++d) {
-    const double *ch = tree + ((uint64_t(2) << d) - 1);
-    const double l = ch[2 * k], rr = ch[2 * k + 1];
-    if (go_left(r, l, rr)) {
-      k = 2 * k;
-    } else {
-      r = __dsub_rn(r, l);
-      k = 2 * k + 1;
-    }
-  }
-  leaf[s] = uint32_t(k);
-  resid[s] = r;
-  atomicAdd(&count[k], 1u);
-}
-
-// Exclusive scan of the per-leaf counts (one block; leaves <= 2^22): 1024
-// counts per step, read coalesced, scanned with warp shuffles.
-__global__ void __launch_bounds__(1024) count_scan_kernel(const uint32_t *__restrict__ count, uint32_t nleaves,
-                                                          uint32_t *__restrict__ offset,
-                                                          uint32_t *__restrict__ cursor) {
-  __shared__ uint32_t wsum[32];
-  __shared__ uint32_t total;
-  const uint32_t lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
-  uint32_t base = 0;
-  for (uint32_t t0 = 0; t0 < nleaves; t0 += 1024) {
-    const uint32_t i = t0 + threadIdx.x;
-    const uint32_t v = i < nleaves ? count[i] : 0u;
-    uint32_t x = v;  // inclusive scan within the warp
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-      if (lane >= uint32_t(o)) x += y;
-    }
-    if (lane == 31) wsum[w] = x;
-    __syncthreads();
-    if (w == 0) {
-      const uint32_t sw = wsum[lane];
-      uint32_t y = sw;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t z = __shfl_up_sync(0xffffffffu, y, o);
-        if (lane >= uint32_t(o)) y += z;
-      }
-      wsum[lane] = y - sw;  // exclusive over warps
-      if (lane == 31) total = y;
-    }
-    __syncthreads();
-    const uint32_t excl = base + wsum[w] + x - v;
-    if (i < nleaves) {
-      offset[i] = excl;
-      cursor[i] = excl;
-    }
-    base += total;
-    __syncthreads();
-  }
-}
-
-__global__ void shot_bucket_kernel(const uint32_t *__restrict__ leaf, uint64_t shots, uint32_t *__restrict__ cursor,
-                                   uint32_t *__restrict__ order) {
-  const uint64_t s = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (s >= shots) return;
-  order[atomicAdd(&cursor[leaf[s]], 1u)] = uint32_t(s);
-}
-
-// One block per leaf with shots: the leaf's tree in shared memory (the same
-// sums as leaf_sum_kernel), then each of its shots walks it to an amplitude.
+// Four consecutive amplitudes' probabilities (zero past the end of the state).
 template <typename C2>
-__global__ void __launch_bounds__(kLeafThreads) leaf_sample_kernel(const C2 *__restrict__ psi, uint64_t N,
-                                                                   uint32_t nleaves, const uint32_t *__restrict__ count,
-                                                                   const uint32_t *__restrict__ offset,
-                                                                   const uint32_t *__restrict__ order,
-                                                                   const double *__restrict__ resid,
-                                                                   uint64_t *__restrict__ out) {
-  extern __shared__ double t[];  // level k (2^k nodes) at t + 2^k - 1; leaves' amplitudes at depth 12
-  for (uint32_t lf = blockIdx.x; lf < nleaves; lf += gridDim.x) {
-    const uint32_t c = count[lf];
-    if (c == 0) continue;
-    const uint64_t base = uint64_t(lf) * kLeafAmps;
-    double *amps = t + (kLeafAmps - 1);
-    for (uint32_t j = threadIdx.x; j < kLeafAmps; j += blockDim.x) amps[j] = prob(psi, base + j, N);
-    __syncthreads();
-    for (int d = kLeafBits - 1; d >= 0; --d) {
-      const uint32_t nodes = 1u << d;
-      double *lv = t + (nodes - 1), *ch = t + (2 * nodes - 1);
-      for (uint32_t k = threadIdx.x; k < nodes; k += blockDim.x) lv[k] = __dadd_rn(ch[2 * k], ch[2 * k + 1]);
-      __syncthreads();
+__device__ __forceinline__ void prob4(const C2 *__restrict__ psi, uint64_t i, uint64_t N, double (&p)[4]) {
+  if constexpr (sizeof(C2) == 8) {
+    if (i + 4 <= N) {
+      const float4 *q = reinterpret_cast<const float4 *>(psi + i);
+      const float4 x = q[0], y = q[1];
+      p[0] = prob_of(make_float2(x.x, x.y));
+      p[1] = prob_of(make_float2(x.z, x.w));
+      p[2] = prob_of(make_float2(y.x, y.y));
+      p[3] = prob_of(make_float2(y.z, y.w));
+      return;
     }
-    const uint32_t o = offset[lf];
-    for (uint32_t q = threadIdx.x; q < c; q += blockDim.x) {
-      const uint32_t s = order[o + q];
-      double r = resid[s];
-      uint32_t k = 0;
-      for (int d = 0; d < kLeafBits; ++d) {
-        const double *ch = t + ((2u << d) - 1);
-        const double l = ch[2 * k], rr = ch[2 * k + 1];
-        if (go_left(r, l, rr)) {
-          k = 2 * k;
-        } else {
-          r = __dsub_rn(r, l);
-          k = 2 * k + 1;
+  }
+#pragma unroll
+  for (int j = 0; j < 4; ++j) p[j] = i + j < N ? prob_of(psi[i + j]) : 0.0;
+}
+
+// One warp per `per_warp` (1..32) shots.  First every lane walks one shot down
+// the stored tree (one 16-byte pair of children per level; the warp's 32 walks
+// overlap), then the warp serves its shots one by one: lane l holds amplitudes
+// 4l..4l+3 of the shot's 128-amplitude node, the five levels above them are
+// lane pairs as in node_sum_kernel, and the walk goes on in registers.
+// EXTRA > 0 (more than 30 qubits): the stored nodes hold 2^EXTRA runs of 128
+// amplitudes, whose sums are rebuilt first.
+// A shot reads 128 amplitudes, wherever it falls; before, each leaf of 2^12
+// amplitudes that any shot fell into was read and summed again by a block, for
+// many shots the whole state a second time, after a counting sort of the
+// shots by leaf.  10^6 shots of 28 qubits complex128 on B200: 424 us and 5 us
+// for the tree's upper levels (2 GB of runs: 0.73 of the copy bandwidth),
+// before 1760 us and 140 us for the sort and the upper levels; the first pass
+// 681 us (0.97 of the copy bandwidth; 602 us without storing the lower levels).
+template <typename C2, int EXTRA>
+__global__ void __launch_bounds__(256) shot_kernel(const C2 *__restrict__ psi, uint32_t n,
+                                                   const double *__restrict__ tree, const double *__restrict__ u,
+                                                   uint64_t shots, uint32_t per_warp, uint64_t *__restrict__ out) {
+  constexpr unsigned kAll = 0xffffffffu;
+  const uint64_t N = uint64_t(1) << n;
+  const uint32_t node = kNodeBits + EXTRA;
+  const uint32_t depth = n > node ? n - node : 0;
+  const uint32_t lane = threadIdx.x & 31u;
+  const uint64_t first = ((uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5) * per_warp;
+  if (first >= shots) return;  // uniform over the warp
+  const uint32_t mine = uint32_t(shots - first < per_warp ? shots - first : per_warp);
+  double r = 0.0;
+  uint64_t k = 1;
+  if (lane < mine) {
+    r = __dmul_rn(u[first + lane], tree[1]);
+    for (uint32_t d = 0; d < depth; ++d) {
+      const double2 c = reinterpret_cast<const double2 *>(tree)[k];
+      k = 2 * k;
+      if (!go_left(r, c.x, c.y)) {
+        r = __dsub_rn(r, c.x);
+        ++k;
+      }
+    }
+  }
+  const uint64_t leaf = (k - (uint64_t(1) << depth)) << node;
+  for (uint32_t j = 0; j < mine; ++j) {
+    uint64_t base = __shfl_sync(kAll, leaf, j);
+    double rr = __shfl_sync(kAll, r, j);
+    double p[4];
+    if constexpr (EXTRA > 0) {
+      constexpr int B = 1 << EXTRA;
+      double t[2 * B];  // heap of the node's 128-amplitude runs
+#pragma unroll 1
+      for (int b = 0; b < B; ++b) {
+        prob4(psi, base + uint64_t(b) * 128 + 4 * lane, N, p);
+        double s = __dadd_rn(__dadd_rn(p[0], p[1]), __dadd_rn(p[2], p[3]));
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) s = __dadd_rn(s, __shfl_xor_sync(kAll, s, o));
+        t[B + b] = s;
+      }
+      for (int i = B - 1; i >= 1; --i) t[i] = __dadd_rn(t[2 * i], t[2 * i + 1]);
+      int at = 1;
+#pragma unroll 1
+      for (int e = 0; e < EXTRA; ++e) {
+        const double l = t[2 * at], q = t[2 * at + 1];
+        at = 2 * at;
+        if (!go_left(rr, l, q)) {
+          rr = __dsub_rn(rr, l);
+          ++at;
         }
       }
-      out[s] = base + k;
+      base += uint64_t(at - B) * 128;
     }
-    __syncthreads();
+    prob4(psi, base + 4 * lane, N, p);
+    const double lo = __dadd_rn(p[0], p[1]), hi = __dadd_rn(p[2], p[3]);
+    // sum[e]: the run of 2^e lanes this lane belongs to.
+    double sum[5];
+    sum[0] = __dadd_rn(lo, hi);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) sum[e + 1] = __dadd_rn(sum[e], __shfl_xor_sync(kAll, sum[e], 1 << e));
+    uint32_t at = 0;  // first lane of the node walked to
+#pragma unroll
+    for (int e = 4; e >= 0; --e) {
+      const double l = __shfl_sync(kAll, sum[e], at), q = __shfl_sync(kAll, sum[e], at + (1u << e));
+      if (!go_left(rr, l, q)) {
+        rr = __dsub_rn(rr, l);
+        at += 1u << e;
+      }
+    }
+    if (lane == at) {
+      uint32_t a = 0;
+      double l = p[0], q = p[1];
+      if (!go_left(rr, lo, hi)) {
+        rr = __dsub_rn(rr, lo);
+        a = 2;
+        l = p[2];
+        q = p[3];
+      }
+      if (!go_left(rr, l, q)) ++a;
+      out[first + j] = base + 4 * lane + a;
+    }
   }
 }
 
@@ -429,13 +463,10 @@ int fail(int code, const std::string &msg) { return sq_detail_fail(code, msg.c_s
 
 size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 
-// Scratch bytes of sample_impl: the upper tree, per-leaf counts / offsets /
-// cursors, per-shot leaf, residual and bucket order.
-size_t sample_scratch_bytes(uint32_t n, uint64_t shots) {
-  const uint32_t depth = n > uint32_t(kLeafBits) ? n - kLeafBits : 0;
-  const uint64_t nleaves = uint64_t(1) << depth;
-  return align256((2 * nleaves - 1) * sizeof(double)) + 3 * align256(nleaves * sizeof(uint32_t)) +
-         2 * align256(shots * sizeof(uint32_t)) + align256(shots * sizeof(double));
+// Scratch bytes of sample_impl: the stored tree.
+size_t sample_scratch_bytes(uint32_t n) {
+  const uint32_t node = node_bits(n);
+  return align256((uint64_t(2) << (n > node ? n - node : 0)) * sizeof(double));
 }
 
 // u_ready (optional): an event the shot phase waits for before reading the
@@ -444,53 +475,35 @@ size_t sample_scratch_bytes(uint32_t n, uint64_t shots) {
 template <typename C2>
 int sample_impl(const C2 *psi, uint32_t n, const double *u, uint64_t shots, uint64_t *out, void *scr,
                 cudaStream_t st, cudaEvent_t u_ready = nullptr, const std::function<int()> &before_shots = {}) {
-  const uint64_t N = uint64_t(1) << n;
-  const uint32_t depth = n > uint32_t(kLeafBits) ? n - kLeafBits : 0;
-  const uint64_t nleaves = uint64_t(1) << depth;
-  const size_t b_tree = align256((2 * nleaves - 1) * sizeof(double));
-  const size_t b_leafu = align256(nleaves * sizeof(uint32_t));
-  const size_t b_shot32 = align256(shots * sizeof(uint32_t));
-  char *p = static_cast<char *>(scr);
-  double *tree = reinterpret_cast<double *>(p);
-  p += b_tree;
-  uint32_t *count = reinterpret_cast<uint32_t *>(p);
-  p += b_leafu;
-  uint32_t *offset = reinterpret_cast<uint32_t *>(p);
-  p += b_leafu;
-  uint32_t *cursor = reinterpret_cast<uint32_t *>(p);
-  p += b_leafu;
-  uint32_t *leaf = reinterpret_cast<uint32_t *>(p);
-  p += b_shot32;
-  uint32_t *order = reinterpret_cast<uint32_t *>(p);
-  p += b_shot32;
-  double *resid = reinterpret_cast<double *>(p);
-
-  leaf_sum_kernel<C2><<<unsigned(nleaves), kLeafThreads, 0, st>>>(psi, N, tree + (nleaves - 1));
+  double *tree = static_cast<double *>(scr);
+  const uint32_t node = node_bits(n);
+  const uint32_t blocks_log = n > uint32_t(kBlockBits) ? n - kBlockBits : 0;
+  node_sum_kernel<C2><<<1u << blocks_log, kTreeThreads, 0, st>>>(psi, n, node, tree);
   RQ_CUDA(cudaGetLastError());
-  if (depth) upper_tree_kernel<<<1, 1024, 0, st>>>(tree, depth);
-  RQ_CUDA(cudaGetLastError());
-  RQ_CUDA(cudaMemsetAsync(count, 0, nleaves * sizeof(uint32_t), st));
+  for (uint32_t from = blocks_log; from > 0;) {
+    const uint32_t lv = std::min(from, kUpperLevels);
+    upper_tree_kernel<<<1u << (from - lv), 1024, 0, st>>>(tree, from, lv);
+    RQ_CUDA(cudaGetLastError());
+    from -= lv;
+  }
   if (before_shots) {
     const int rc = before_shots();
     if (rc != SQ_OK) return rc;
   }
   if (u_ready) RQ_CUDA(cudaStreamWaitEvent(st, u_ready, 0));
-  const unsigned sb = unsigned((shots + 255) / 256);
-  shot_descend_kernel<<<sb, 256, 0, st>>>(tree, depth, u, shots, leaf, resid, count);
-  RQ_CUDA(cudaGetLastError());
-  count_scan_kernel<<<1, 1024, 0, st>>>(count, uint32_t(nleaves), offset, cursor);
-  RQ_CUDA(cudaGetLastError());
-  shot_bucket_kernel<<<sb, 256, 0, st>>>(leaf, shots, cursor, order);
-  RQ_CUDA(cudaGetLastError());
-  const size_t smem = (2 * size_t(kLeafAmps) - 1) * sizeof(double);
-  RQ_CUDA(cudaFuncSetAttribute(leaf_sample_kernel<C2>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-  int sms = 0, dev = 0, per_sm = 0;
-  RQ_CUDA(cudaGetDevice(&dev));
-  RQ_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  RQ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, leaf_sample_kernel<C2>, kLeafThreads, smem));
-  const unsigned grid = unsigned(std::min<uint64_t>(nleaves, uint64_t(sms) * uint64_t(std::max(per_sm, 1))));
-  leaf_sample_kernel<C2><<<grid, kLeafThreads, smem, st>>>(psi, N, uint32_t(nleaves), count, offset, order,
-                                                           resid, out);
+  // Shots per warp: as many as leave a warp for every slot of the GPU, at most
+  // 32 (a warp serves its shots one after the other).
+  uint32_t per_warp = 32;
+  while (per_warp > 1 && shots / per_warp < 148 * 64) per_warp >>= 1;
+  const uint64_t warps = (shots + per_warp - 1) / per_warp;
+  const unsigned grid = unsigned((warps + 7) / 8);
+  switch (node - kNodeBits) {
+    case 0: shot_kernel<C2, 0><<<grid, 256, 0, st>>>(psi, n, tree, u, shots, per_warp, out); break;
+    case 1: shot_kernel<C2, 1><<<grid, 256, 0, st>>>(psi, n, tree, u, shots, per_warp, out); break;
+    case 2: shot_kernel<C2, 2><<<grid, 256, 0, st>>>(psi, n, tree, u, shots, per_warp, out); break;
+    case 3: shot_kernel<C2, 3><<<grid, 256, 0, st>>>(psi, n, tree, u, shots, per_warp, out); break;
+    default: shot_kernel<C2, 4><<<grid, 256, 0, st>>>(psi, n, tree, u, shots, per_warp, out);
+  }
   RQ_CUDA(cudaGetLastError());
   return SQ_OK;
 }
@@ -506,9 +519,9 @@ int sq_sample(sq_state *s, const double *uniforms_device, uint64_t shots, uint64
   const int rc = sq_flush(s, stream);
   if (rc != SQ_OK || shots == 0) return rc;
   const uint32_t n = sq_state_num_qubits(s);
-  if (n > uint32_t(kLeafBits) + 22) return fail(SQ_ERR_UNSUPPORTED, "sq_sample: more than 34 qubits");
+  if (n > 34) return fail(SQ_ERR_UNSUPPORTED, "sq_sample: more than 34 qubits");
   void *scr = nullptr;
-  const int sc = sq_detail_state_scratch(s, sample_scratch_bytes(n, shots), &scr);
+  const int sc = sq_detail_state_scratch(s, sample_scratch_bytes(n), &scr);
   if (sc != SQ_OK) return sc;
   if (sq_state_dtype(s) == SQ_C64)
     return sample_impl(static_cast<const float2 *>(sq_state_data(s)), n, uniforms_device, shots, out_device, scr, st);
@@ -523,11 +536,11 @@ int sq_sample_host(sq_state *s, const double *uniforms, uint64_t shots, uint64_t
   int rc = sq_flush(s, stream);
   if (rc != SQ_OK || shots == 0) return rc;
   const uint32_t n = sq_state_num_qubits(s);
-  if (n > uint32_t(kLeafBits) + 22) return fail(SQ_ERR_UNSUPPORTED, "sq_sample_host: more than 34 qubits");
+  if (n > 34) return fail(SQ_ERR_UNSUPPORTED, "sq_sample_host: more than 34 qubits");
   // The state's scratch holds the uniforms and the indices, then the sampler's own scratch.
   const size_t b_u = align256(shots * sizeof(double)), b_o = align256(shots * sizeof(uint64_t));
   void *scr = nullptr;
-  rc = sq_detail_state_scratch(s, b_u + b_o + sample_scratch_bytes(n, shots), &scr);
+  rc = sq_detail_state_scratch(s, b_u + b_o + sample_scratch_bytes(n), &scr);
   if (rc != SQ_OK) return rc;
   char *p = static_cast<char *>(scr);
   double *du = reinterpret_cast<double *>(p);
