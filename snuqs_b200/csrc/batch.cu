@@ -22,6 +22,7 @@
 
 #include "../../include/snuqs_b200.h"
 #include "adjoint_plan.h"
+#include "batch_energy.cuh"
 #include "batch_kernels.cuh"
 #include "host_ops.h"
 #include "jit.h"
@@ -122,14 +123,16 @@ struct sq_batch {
   int device = 0;
   int keep = 0;
   std::vector<sq::PauliParams> hams;
+  std::vector<sq::PauliTilePlan> ham_tiles;  // the same sums, for the energy pass of streamed states
   std::vector<uint32_t> ham_n;
   std::vector<Circ> circs;
-  DevBuf d_pool, d_plans, d_table, d_hams, d_energy, d_counter, d_occ, d_def, d_part;
+  DevBuf d_pool, d_plans, d_table, d_hams, d_tiles, d_energy, d_counter, d_occ, d_def, d_part;
   HostBuf h_plans, h_table, h_energy, h_occ, h_def;
   std::vector<uint32_t> deferred;  // table positions whose energy the grid-wide pass computes
   uint32_t nitems = 0;              // work items of that pass
+  uint32_t tile_terms = 0, tile_groups = 0;  // largest pass of its Hamiltonians
   size_t def_words = 0;             // staged words: deferred circuits, item offsets
-  size_t hams_uploaded = 0;
+  size_t hams_uploaded = 0, tiles_uploaded = 0;
   std::vector<uint64_t> state_off;  // per circuit id; ~0 when not kept
   std::vector<uint32_t> order;      // sorted position -> circuit id
   cudaGraphExec_t graph = nullptr;
@@ -169,7 +172,8 @@ struct sq_batch {
 namespace {
 
 // Pauli-string sum -> grouped expectation parameters (as sq_expect_pauli).
-int build_pauli(uint32_t n, const char *paulis, const double *w, uint32_t nt, sq::PauliParams &P) {
+int build_pauli(uint32_t n, const char *paulis, const double *w, uint32_t nt, sq::PauliParams &P,
+                sq::PauliTilePlan &T) {
   if (nt > uint32_t(sq::kMaxTerms)) return fail(SQ_ERR_UNSUPPORTED, "batch: > 1024 Pauli terms");
   std::vector<uint64_t> xm(nt), zym(nt);
   std::vector<int> ny(nt);
@@ -211,6 +215,10 @@ int build_pauli(uint32_t n, const char *paulis, const double *w, uint32_t nt, sq
     g.t1 = k;
     pos = end;
   }
+  // A batch's circuits fill the GPU together: as few passes as possible.
+  std::memset(&T, 0, sizeof(T));
+  if (sq::plan_pauli_tiles(T, n, idx.data(), nt, 0, xm.data(), zym.data(), ny.data(), w, 1) != nt)
+    return fail(SQ_ERR_UNSUPPORTED, "batch: the Pauli terms do not fit one plan");
   return SQ_OK;
 }
 
@@ -741,6 +749,12 @@ int run_impl(sq_batch *b, double *energies, cudaStream_t st) {
                         cudaMemcpyHostToDevice));
     b->hams_uploaded = b->hams.size();
   }
+  if (b->tiles_uploaded != b->ham_tiles.size()) {
+    const size_t bytes = b->ham_tiles.size() * sizeof(sq::PauliTilePlan);
+    if (int s = b->d_tiles.ensure(bytes)) return s;
+    SQB_CUDA(cudaMemcpy(b->d_tiles.p, b->ham_tiles.data(), bytes, cudaMemcpyHostToDevice));
+    b->tiles_uploaded = b->ham_tiles.size();
+  }
   // Pinned staging: packed plans and the sorted table.
   auto *tab = static_cast<sq::BatchCircuit *>(b->h_table.p);
   unsigned char *hp = static_cast<unsigned char *>(b->h_plans.p);
@@ -771,15 +785,19 @@ int run_impl(sq_batch *b, double *energies, cudaStream_t st) {
     G.pool_off = tab[G.first].state_off;
     G.plan_off = tab[G.first].plan_off;
   }
-  // Work items of the energy pass: chunks of 2^kEnergyChunkBits pairs.
+  // Work items of the energy pass: (pass, tile) of every deferred circuit.
   // Staged as [deferred | item_off (ndef+1)]; the kernel finds an item's
   // circuit by binary search over item_off.
   {
     std::vector<uint32_t> item_off{0};
+    b->tile_terms = b->tile_groups = 0;
     for (uint32_t k = 0; k < b->deferred.size(); ++k) {
-      const uint32_t n = tab[b->deferred[k]].n;
-      const uint32_t chunks = n - 1 > sq::kEnergyChunkBits ? 1u << (n - 1 - sq::kEnergyChunkBits) : 1u;
-      item_off.push_back(item_off.back() + chunks);
+      const sq::BatchCircuit &t = tab[b->deferred[k]];
+      const sq::PauliTilePlan &T = b->ham_tiles[t.ham];
+      if (T.m != sq::kPauliTileBits) return fail(SQ_ERR_INVALID, "internal: a streamed state below one energy tile");
+      item_off.push_back(item_off.back() + (T.npasses << (T.n - T.m)));
+      b->tile_terms = std::max(b->tile_terms, T.max_terms);
+      b->tile_groups = std::max(b->tile_groups, T.max_groups);
     }
     b->nitems = item_off.back();
     std::vector<uint32_t> staged(b->deferred);
@@ -808,9 +826,13 @@ int run_impl(sq_batch *b, double *energies, cudaStream_t st) {
     SQB_CUDA(cudaEventCreate(&b->ev0));
     SQB_CUDA(cudaEventCreate(&b->ev1));
   }
-  // Grid-wide energy pass over the streamed states: 4 blocks per SM.
+  // Grid-wide energy pass over the streamed states: the resident blocks, 3 per SM.
   uint32_t ndef = uint32_t(b->deferred.size());
-  const uint32_t egrid = uint32_t(std::max<uint64_t>(1, std::min<uint64_t>(b->nitems, uint64_t(sms) * 8)));
+  const uint32_t egrid = uint32_t(std::max<uint64_t>(1, std::min<uint64_t>(b->nitems, uint64_t(sms) * 3)));
+  const uint32_t esmem = sq::pauli_tile_smem(b->tile_terms, b->tile_groups);
+  if (esmem > 48 * 1024)
+    SQB_CUDA(cudaFuncSetAttribute(sq::batch_energy_tiles<Real>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  int(sq::pauli_tile_smem(sq::kPauliMaxTerms, sq::kPauliMaxGroups))));
   if (int s = b->d_part.ensure(std::max<size_t>(b->nitems, 1) * sizeof(double))) return s;
   // (Re)capture the graph when sizes or the stream changed.
   if (!b->graph || b->graph_plan_bytes != plan_bytes || b->graph_ncirc != nc ||
@@ -863,11 +885,9 @@ int run_impl(sq_batch *b, double *energies, cudaStream_t st) {
         const uint32_t *defp = static_cast<const uint32_t *>(b->d_def.p);
         const uint32_t *offp = defp + ndef;
         double *partp = static_cast<double *>(b->d_part.p);
-        const C2 *cpool = poolp;
-        uint32_t nitems = b->nitems;
-        void *gargs[] = {&cpool, &P, &defp, &offp, &ndef, &nitems, &partp};
-        cudaLaunchKernel(reinterpret_cast<const void *>(&sq::batch_energy_grid<Real>), dim3(egrid),
-                         dim3(sq::kReduceThreads), gargs, 0, cs);
+        sq::batch_energy_tiles<Real><<<egrid, sq::kPauliThreads, esmem, cs>>>(
+            poolp, P.circuits, static_cast<const sq::PauliTilePlan *>(b->d_tiles.p), defp, offp, ndef, b->nitems,
+            b->tile_terms, b->tile_groups, partp);
         sq::batch_energy_finalize<<<ndef, sq::kReduceThreads, 0, cs>>>(partp, offp, defp, P.energies);
       }
       cudaEventRecordWithFlags(b->ev1, cs, cudaEventRecordExternal);
@@ -1168,6 +1188,7 @@ int sq_batch_destroy(sq_batch *b) {
   b->d_plans.release();
   b->d_table.release();
   b->d_hams.release();
+  b->d_tiles.release();
   b->d_energy.release();
   b->d_counter.release();
   b->d_occ.release();
@@ -1214,9 +1235,11 @@ int sq_batch_add_hamiltonian(sq_batch *b, uint32_t num_qubits, const char *pauli
                              const double *weights, uint32_t n_terms, uint32_t *ham_id) {
   if (!b || !ham_id || (n_terms && (!paulis || !weights))) return fail(SQ_ERR_INVALID, "null pointer");
   if (num_qubits < 4 || num_qubits > 30) return fail(SQ_ERR_UNSUPPORTED, "batch: 4..30 qubits");
-  sq::PauliParams P;
-  if (int s = build_pauli(num_qubits, paulis, weights, n_terms, P)) return s;
-  b->hams.push_back(P);
+  auto P = std::make_unique<sq::PauliParams>();
+  auto T = std::make_unique<sq::PauliTilePlan>();
+  if (int s = build_pauli(num_qubits, paulis, weights, n_terms, *P, *T)) return s;
+  b->hams.push_back(*P);
+  b->ham_tiles.push_back(*T);
   b->ham_n.push_back(num_qubits);
   *ham_id = uint32_t(b->hams.size() - 1);
   return SQ_OK;

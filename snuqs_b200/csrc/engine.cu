@@ -23,6 +23,7 @@
 #include "engine_internal.h"
 #include "host_ops.h"
 #include "jit.h"
+#include "pauli_tiles.cuh"
 #include "reduce_kernels.cuh"
 #include "sweep_kernels.cuh"
 #include "sweep_registry.h"
@@ -995,69 +996,35 @@ int sq_probabilities(sq_state *s, double *out_device, void *stream) {
   return SQ_OK;
 }
 
-// Groups Pauli terms by (flip mask, Y parity) and runs the expectation
-// kernel over each batch of groups; returns the FP64 sum.
+// Orders Pauli terms by (flip mask, Y parity) and runs the tiled expectation
+// over each plan's worth of groups; returns the FP64 sum.
 static int expect_impl(sq_state *s, const std::vector<uint64_t> &xm,
                        const std::vector<uint64_t> &zym, const std::vector<int> &ny,
                        const std::vector<double> &w, double *out, cudaStream_t st) {
   SQ_TRY(flush_impl(s, st));
   DeviceInfo di;
   SQ_TRY(device_info(s->device, di));
-  const uint32_t n = s->n;
-  // Sort term indices by (x, parity).
-  std::vector<size_t> idx(xm.size());
-  for (size_t i = 0; i < idx.size(); ++i) idx[i] = i;
-  std::stable_sort(idx.begin(), idx.end(), [&](size_t a, size_t b) {
+  std::vector<uint32_t> idx(xm.size());
+  for (size_t i = 0; i < idx.size(); ++i) idx[i] = uint32_t(i);
+  std::stable_sort(idx.begin(), idx.end(), [&](uint32_t a, uint32_t b) {
     if (xm[a] != xm[b]) return xm[a] < xm[b];
     return (ny[a] & 1) < (ny[b] & 1);
   });
-  const uint64_t pairs = n ? (uint64_t(1) << (n - 1)) : 1;
-  const uint32_t blocks = uint32_t(std::max<uint64_t>(
-      1, std::min<uint64_t>((pairs + sq::kReduceThreads - 1) / sq::kReduceThreads,
-                            uint64_t(di.sms) * 4)));
+  const uint32_t blocks = uint32_t(di.sms) * 3;  // the kernel's resident blocks
   SQ_TRY(ensure_scratch(s, blocks + 1));
-  auto P = std::make_unique<sq::PauliParams>();
+  auto P = std::make_unique<sq::PauliTilePlan>();
+  const uint32_t nterms = uint32_t(idx.size());
+  uint32_t pos = 0;
   bool first_launch = true;
-  size_t pos = 0;
-  while (pos < idx.size() || first_launch) {
-    std::memset(P.get(), 0, sizeof(*P));
-    P->n = n;
-    uint32_t nt = 0;
-    while (pos < idx.size()) {
-      const size_t i0 = idx[pos];
-      size_t end = pos;
-      while (end < idx.size() && xm[idx[end]] == xm[i0] && ((ny[idx[end]] & 1) == (ny[i0] & 1)))
-        ++end;
-      const size_t cnt = end - pos;
-      if (P->ngroups >= uint32_t(sq::kMaxGroups) || nt + cnt > size_t(sq::kMaxTerms)) {
-        if (nt == 0) return fail(SQ_ERR_UNSUPPORTED, "more than %d terms share one Pauli group",
-                                 sq::kMaxTerms);
-        break;
-      }
-      sq::PauliGroup &g = P->g[P->ngroups++];
-      g.x = xm[i0];
-      g.odd = ny[i0] & 1;
-      g.t0 = nt;
-      for (size_t e = pos; e < end; ++e) {
-        const size_t t = idx[e];
-        // (-i)^ny folded into a real factor: even ny -> Re((-i)^ny) = (-1)^(ny/2);
-        // odd ny -> -Im((-i)^ny) = (-1)^((ny-1)/2).
-        const int half = ny[t] / 2;
-        const double sign = (half & 1) ? -1.0 : 1.0;
-        P->zy[nt] = zym[t];
-        P->f[nt] = w[t] * sign;
-        ++nt;
-      }
-      g.t1 = nt;
-      pos = end;
-    }
-    if (s->dtype == SQ_C64)
-      sq::pauli_expect_kernel<float><<<blocks, sq::kReduceThreads, 0, st>>>(
-          static_cast<const float2 *>(s->data), *P, s->scratch, first_launch ? 0 : 1);
-    else
-      sq::pauli_expect_kernel<double><<<blocks, sq::kReduceThreads, 0, st>>>(
-          static_cast<const double2 *>(s->data), *P, s->scratch, first_launch ? 0 : 1);
-    SQ_CUDA(cudaGetLastError());
+  while (pos < nterms || first_launch) {
+    const uint32_t next = sq::plan_pauli_tiles(*P, s->n, idx.data(), nterms, pos, xm.data(), zym.data(), ny.data(),
+                                               w.data(), blocks);
+    if (next == pos && nterms)
+      return fail(SQ_ERR_UNSUPPORTED, "more than %d terms share one Pauli group", sq::kMaxTerms);
+    pos = next;
+    SQ_CUDA(s->dtype == SQ_C64
+                ? sq::launch_pauli_tiles<float>(s->data, *P, s->scratch, blocks, !first_launch, st)
+                : sq::launch_pauli_tiles<double>(s->data, *P, s->scratch, blocks, !first_launch, st));
     first_launch = false;
   }
   sq::finalize_sum_kernel<<<1, sq::kReduceThreads, 0, st>>>(s->scratch, blocks, s->scratch + blocks);

@@ -23,7 +23,7 @@
 // (16 KiB of FP64 partials), at most 1024 Pauli terms and 256 distinct
 // (X/Y mask, Y parity) groups per call.  Larger requests are rejected.
 // Each call stages the grouped terms on the calling thread's stack (about
-// 45 KiB: the kernel's parameter block and four term arrays).
+// 50 KiB: the kernel's parameter block and four term arrays).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -31,6 +31,7 @@
 #include <mutex>
 
 #include "../../include/snuqs_b200.h"
+#include "pauli_tiles.cuh"
 #include "reduce_kernels.cuh"
 
 int sq_detail_fail(int code, const char *msg);  // engine.cu: sets sq_last_error()
@@ -140,46 +141,22 @@ extern "C" int sq_expect_pauli_noalloc(const void *state, uint32_t num_qubits, i
     if (xm[a] != xm[b]) return xm[a] < xm[b];
     return (ny[a] & 1) < (ny[b] & 1);
   });
-  sq::PauliParams P;  // 22 KiB on the stack
-  std::memset(&P, 0, sizeof(P));
-  P.n = n;
-  uint32_t nt = 0;
-  for (uint32_t pos = 0; pos < n_terms;) {
-    const uint32_t i0 = idx[pos];
-    uint32_t end = pos;
-    while (end < n_terms && xm[idx[end]] == xm[i0] && (ny[idx[end]] & 1) == (ny[i0] & 1)) ++end;
-    if (P.ngroups >= uint32_t(sq::kMaxGroups))
-      return fail(SQ_ERR_UNSUPPORTED,
-                  "sq_expect_pauli_noalloc: more than 256 distinct Pauli groups");
-    sq::PauliGroup &g = P.g[P.ngroups++];
-    g.x = xm[i0];
-    g.odd = ny[i0] & 1;
-    g.t0 = nt;
-    for (uint32_t k = pos; k < end; ++k) {
-      const uint32_t t = idx[k];
-      // (-i)^ny folded into a real factor (see reduce_kernels.cuh).
-      P.zy[nt] = zym[t];
-      P.f[nt] = weights[t] * (((ny[t] / 2) & 1) ? -1.0 : 1.0);
-      ++nt;
-    }
-    g.t1 = nt;
-    pos = end;
-  }
-
-  const uint64_t pairs = uint64_t(1) << (n - 1);
-  const uint32_t blocks = uint32_t(std::max<uint64_t>(
-      1, std::min<uint64_t>({(pairs + sq::kReduceThreads - 1) / sq::kReduceThreads,
-                             uint64_t(sms) * 4, uint64_t(kNoAllocMaxBlocks)})));
+  // Every term in one plan (at most 256 groups: checked here).
+  uint32_t groups = 0;
+  for (uint32_t t = 0; t < n_terms; ++t)
+    if (t == 0 || xm[idx[t]] != xm[idx[t - 1]] || (ny[idx[t]] & 1) != (ny[idx[t - 1]] & 1)) ++groups;
+  if (groups > sq::kPauliMaxGroups)
+    return fail(SQ_ERR_UNSUPPORTED,
+                "sq_expect_pauli_noalloc: more than 256 distinct Pauli groups");
+  const uint32_t blocks = std::min(uint32_t(sms) * 3, uint32_t(kNoAllocMaxBlocks));
+  sq::PauliTilePlan P;  // 26 KiB on the stack
+  if (sq::plan_pauli_tiles(P, n, idx, n_terms, 0, xm, zym, ny, weights, blocks) != n_terms)
+    return fail(SQ_ERR_UNSUPPORTED, "sq_expect_pauli_noalloc: the terms do not fit one plan");
   auto s = static_cast<cudaStream_t>(stream);
   // accumulate = 0: every used partial slot is overwritten, so the previous
   // call's contents need no clearing.
-  if (dtype == SQ_C64)
-    sq::pauli_expect_kernel<float><<<blocks, sq::kReduceThreads, 0, s>>>(
-        static_cast<const float2 *>(state), P, partials, 0);
-  else
-    sq::pauli_expect_kernel<double><<<blocks, sq::kReduceThreads, 0, s>>>(
-        static_cast<const double2 *>(state), P, partials, 0);
-  e = cudaGetLastError();
+  e = dtype == SQ_C64 ? sq::launch_pauli_tiles<float>(state, P, partials, blocks, 0, s)
+                      : sq::launch_pauli_tiles<double>(state, P, partials, blocks, 0, s);
   if (e != cudaSuccess) return fail(SQ_ERR_CUDA, cudaGetErrorString(e));
   // Fixed-order sum of the partials into the caller's output (deterministic).
   sq::finalize_sum_kernel<<<1, sq::kReduceThreads, 0, s>>>(partials, blocks, out_device);

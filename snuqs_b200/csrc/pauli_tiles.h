@@ -1,0 +1,181 @@
+// Pauli-sum expectations by tiles: the plan the host makes and the kernels
+// (pauli_tiles.cuh) run.
+//
+// A Pauli string with flip mask x pairs amplitude i with i ^ x, so a group of
+// strings of one mask needs one read of the state when the pairs are fetched
+// from memory.  Flip masks form a vector space over GF(2): a tile that holds
+// a coset base ^ span(v_1 .. v_k) of index space holds both amplitudes of
+// every pair of EVERY group whose mask lies in the span.  A pass therefore
+// collects groups while their masks fit a span of kPauliTileBits dimensions
+// (the kPauliLowBits lowest index bits, so that a tile is made of 128-byte
+// runs of complex128 amplitudes, and eight more generators), and the state is
+// read once per pass: 64 random strings of 25 qubits take 8 passes instead
+// of 64 reads.
+#pragma once
+#include <stdint.h>
+
+namespace sq {
+
+constexpr uint32_t kPauliTileBits = 11;
+constexpr uint32_t kPauliLowBits = 3;
+constexpr uint32_t kPauliGens = kPauliTileBits - kPauliLowBits;
+constexpr uint32_t kPauliMaxTerms = 1024;
+constexpr uint32_t kPauliMaxGroups = 256;
+constexpr uint32_t kPauliMaxPasses = 40;
+
+struct alignas(8) PauliTileGroup {
+  uint16_t c;       // flip mask in tile coordinates (0: diagonal)
+  uint16_t odd;     // odd number of Y: the pair's imaginary part
+  uint16_t t0, t1;  // terms
+};
+
+struct PauliTilePass {
+  uint64_t gen[kPauliGens];    // global index vector of tile bit low + i
+  uint8_t pivot[kPauliGens];   // ascending bits the tile base has clear
+  uint16_t g0, g1;             // groups
+};
+
+// Tile index j stands for global index base ^ (j's low bits) ^ gens of its
+// other bits; base runs over the indices with the low and pivot bits clear.
+struct PauliTilePlan {
+  uint32_t n;
+  uint32_t m, low;   // tile bits, low bits (both at most n)
+  uint32_t npasses;
+  uint32_t max_terms, max_groups;  // of any pass (shared-memory sizes)
+  PauliTilePass pass[kPauliMaxPasses];
+  PauliTileGroup group[kPauliMaxGroups];
+  uint64_t zy[kPauliMaxTerms];   // Z-or-Y mask (global index bits)
+  double f[kPauliMaxTerms];      // weight and phase
+  // Z-or-Y mask in tile coordinates (bits 0..10), and at bit 16 + r its parity
+  // on tile row r (tile bits 8 and up).
+  uint32_t zt[kPauliMaxTerms];
+};
+
+// Dynamic shared memory of the kernels for passes of at most these sizes:
+// the tile as complex doubles, the groups, per term a weight and a word.
+constexpr uint32_t pauli_tile_smem(uint32_t terms, uint32_t groups) {
+  return (16u << kPauliTileBits) + groups * 8u + terms * 12u;
+}
+
+// Plans the groups that start at term position `pos` of the term order idx
+// (sorted by flip mask, then parity of the Y count): as many groups as the
+// plan holds, at least one.  xm / zym / ny / w: per term the flip mask,
+// Z-or-Y mask, Y count and weight.  `items`: work items (tile x pass) that
+// fill the GPU; a state of few tiles gets more passes of fewer groups.
+// Returns the position after the last planned term; `pos` itself when one
+// group has more than kPauliMaxTerms terms.  Allocates nothing.
+template <class Index>
+uint32_t plan_pauli_tiles(PauliTilePlan &P, uint32_t n, const Index *idx, uint32_t nterms, uint32_t pos,
+                          const uint64_t *xm, const uint64_t *zym, const int *ny, const double *w,
+                          uint32_t items) {
+  P.n = n;
+  P.m = n < kPauliTileBits ? n : kPauliTileBits;
+  P.low = n < kPauliLowBits ? n : kPauliLowBits;
+  P.npasses = P.max_terms = P.max_groups = 0;
+  // Groups [first, last) of the term order.
+  uint16_t first[kPauliMaxGroups], last[kPauliMaxGroups];
+  bool taken[kPauliMaxGroups];
+  uint32_t ngroups = 0;
+  const uint32_t base = pos;
+  while (pos < nterms && ngroups < kPauliMaxGroups) {
+    uint32_t end = pos;
+    while (end < nterms && xm[idx[end]] == xm[idx[pos]] && (ny[idx[end]] & 1) == (ny[idx[pos]] & 1)) ++end;
+    if (end - base > kPauliMaxTerms) break;
+    first[ngroups] = uint16_t(pos - base);
+    last[ngroups] = uint16_t(end - base);
+    taken[ngroups++] = false;
+    pos = end;
+  }
+  const uint64_t lowmask = (uint64_t(1) << P.low) - 1;
+  const uint32_t gens = P.m - P.low;
+  const uint64_t tiles = uint64_t(1) << (n - P.m);
+  // Groups per pass: all that fit when the tiles alone fill the GPU.
+  uint32_t cap = kPauliMaxGroups;
+  if (tiles < items && ngroups) {
+    uint64_t passes = (items + tiles - 1) / tiles;
+    if (passes > 32) passes = 32;
+    cap = uint32_t((ngroups + passes - 1) / passes);
+  }
+  uint32_t ng = 0, nt = 0;
+  for (uint32_t left = ngroups; left;) {
+    if (P.npasses == kPauliMaxPasses) return base;  // cannot happen: see kPauliMaxPasses
+    PauliTilePass &S = P.pass[P.npasses++];
+    uint64_t gen[kPauliGens];
+    uint32_t piv[kPauliGens], dim = 0;
+    // gen stays reduced: bit piv[i] is set in gen[i] only.
+    auto add = [&](uint64_t x) -> bool {
+      for (uint32_t i = 0; i < dim; ++i)
+        if ((x >> piv[i]) & 1) x ^= gen[i];
+      if (!x) return true;
+      if (dim == gens) return false;
+      uint32_t p = 0;
+      while (!((x >> p) & 1)) ++p;
+      for (uint32_t i = 0; i < dim; ++i)
+        if ((gen[i] >> p) & 1) gen[i] ^= x;
+      gen[dim] = x;
+      piv[dim++] = p;
+      return true;
+    };
+    uint16_t member[kPauliMaxGroups];
+    uint32_t nm = 0;
+    for (uint32_t g = 0; g < ngroups && nm < cap; ++g)
+      if (!taken[g] && add(xm[idx[base + first[g]]] & ~lowmask)) {
+        taken[g] = true;
+        member[nm++] = uint16_t(g);
+      }
+    left -= nm;
+    for (uint32_t b = P.low; dim < gens; ++b) add(uint64_t(1) << b);  // fill with the lowest free bits
+    // Tile bits in ascending pivot order.
+    for (uint32_t i = 0; i < gens; ++i)
+      for (uint32_t j = i + 1; j < gens; ++j)
+        if (piv[j] < piv[i]) {
+          const uint32_t tp = piv[i];
+          piv[i] = piv[j];
+          piv[j] = tp;
+          const uint64_t tg = gen[i];
+          gen[i] = gen[j];
+          gen[j] = tg;
+        }
+    for (uint32_t i = 0; i < kPauliGens; ++i) {
+      S.gen[i] = i < gens ? gen[i] : 0;
+      S.pivot[i] = uint8_t(i < gens ? piv[i] : 0);
+    }
+    S.g0 = uint16_t(ng);
+    const uint32_t t_begin = nt;
+    for (uint32_t k = 0; k < nm; ++k) {
+      const uint32_t g = member[k], i0 = idx[base + first[g]];
+      const uint64_t x = xm[i0];
+      PauliTileGroup &G = P.group[ng++];
+      uint64_t rest = x;
+      uint32_t c = 0;
+      for (uint32_t i = 0; i < gens; ++i)
+        if ((x >> piv[i]) & 1) {
+          c |= 1u << (P.low + i);
+          rest ^= gen[i];
+        }
+      G.c = uint16_t(c | uint32_t(rest));
+      G.odd = uint16_t(ny[i0] & 1);
+      G.t0 = uint16_t(nt);
+      for (uint32_t e = first[g]; e < last[g]; ++e) {
+        const uint32_t t = idx[base + e];
+        P.zy[nt] = zym[t];
+        // (-i)^ny folded into a real factor: even ny (-1)^(ny/2), odd ny
+        // (-1)^((ny-1)/2) for the imaginary part; a pair counts twice.
+        P.f[nt] = w[t] * (((ny[t] / 2) & 1) ? -1.0 : 1.0) * (x ? 2.0 : 1.0);
+        uint32_t zt = uint32_t(zym[t] & lowmask);
+        for (uint32_t i = 0; i < gens; ++i)
+          if (__builtin_popcountll(gen[i] & zym[t]) & 1) zt |= 1u << (P.low + i);
+        for (uint32_t r = 0; r < 8; ++r)
+          if (__builtin_popcount((r << 8) & zt) & 1) zt |= 1u << (16 + r);
+        P.zt[nt++] = zt;
+      }
+      G.t1 = uint16_t(nt);
+    }
+    S.g1 = uint16_t(ng);
+    if (nt - t_begin > P.max_terms) P.max_terms = nt - t_begin;
+    if (nm > P.max_groups) P.max_groups = nm;
+  }
+  return pos;
+}
+
+}  // namespace sq
