@@ -826,9 +826,9 @@ int run_impl(sq_batch *b, double *energies, cudaStream_t st) {
     SQB_CUDA(cudaEventCreate(&b->ev0));
     SQB_CUDA(cudaEventCreate(&b->ev1));
   }
-  // Grid-wide energy pass over the streamed states: the resident blocks, 3 per SM.
+  // Grid-wide energy pass over the streamed states: the resident blocks, 4 per SM.
   uint32_t ndef = uint32_t(b->deferred.size());
-  const uint32_t egrid = uint32_t(std::max<uint64_t>(1, std::min<uint64_t>(b->nitems, uint64_t(sms) * 3)));
+  const uint32_t egrid = uint32_t(std::max<uint64_t>(1, std::min<uint64_t>(b->nitems, uint64_t(sms) * 4)));
   const uint32_t esmem = sq::pauli_tile_smem(b->tile_terms, b->tile_groups);
   if (esmem > 48 * 1024)
     SQB_CUDA(cudaFuncSetAttribute(sq::batch_energy_tiles<Real>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -887,7 +887,7 @@ int run_impl(sq_batch *b, double *energies, cudaStream_t st) {
         double *partp = static_cast<double *>(b->d_part.p);
         sq::batch_energy_tiles<Real><<<egrid, sq::kPauliThreads, esmem, cs>>>(
             poolp, P.circuits, static_cast<const sq::PauliTilePlan *>(b->d_tiles.p), defp, offp, ndef, b->nitems,
-            b->tile_terms, b->tile_groups, partp);
+            b->tile_terms, partp);
         sq::batch_energy_finalize<<<ndef, sq::kReduceThreads, 0, cs>>>(partp, offp, defp, P.energies);
       }
       cudaEventRecordWithFlags(b->ev1, cs, cudaEventRecordExternal);

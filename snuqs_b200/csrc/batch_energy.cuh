@@ -15,13 +15,13 @@
 namespace sq {
 
 template <typename Real>
-__global__ void __launch_bounds__(kPauliThreads, 3)
+__global__ void __launch_bounds__(kPauliThreads, 4)
     batch_energy_tiles(const typename Vec2<Real>::T *__restrict__ pool, const BatchCircuit *__restrict__ circuits,
                        const PauliTilePlan *__restrict__ plans, const uint32_t *__restrict__ deferred,
                        const uint32_t *__restrict__ item_off, uint32_t ndef, uint32_t nitems, uint32_t max_terms,
-                       uint32_t max_groups, double *__restrict__ partials) {
+                       double *__restrict__ partials) {
   extern __shared__ __align__(16) unsigned char pauli_raw[];
-  PauliShared sh(pauli_raw, max_terms, max_groups);
+  PauliShared sh(pauli_raw, max_terms);
   for (uint32_t w = blockIdx.x; w < nitems; w += gridDim.x) {
     // Deferred circuit k with item_off[k] <= w < item_off[k + 1].
     uint32_t k = 0, end = ndef;

@@ -1010,7 +1010,7 @@ static int expect_impl(sq_state *s, const std::vector<uint64_t> &xm,
     if (xm[a] != xm[b]) return xm[a] < xm[b];
     return (ny[a] & 1) < (ny[b] & 1);
   });
-  const uint32_t blocks = uint32_t(di.sms) * 3;  // the kernel's resident blocks
+  const uint32_t blocks = uint32_t(di.sms) * 4;  // the kernel's resident blocks
   SQ_TRY(ensure_scratch(s, blocks + 1));
   auto P = std::make_unique<sq::PauliTilePlan>();
   const uint32_t nterms = uint32_t(idx.size());

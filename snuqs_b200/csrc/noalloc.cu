@@ -148,7 +148,7 @@ extern "C" int sq_expect_pauli_noalloc(const void *state, uint32_t num_qubits, i
   if (groups > sq::kPauliMaxGroups)
     return fail(SQ_ERR_UNSUPPORTED,
                 "sq_expect_pauli_noalloc: more than 256 distinct Pauli groups");
-  const uint32_t blocks = std::min(uint32_t(sms) * 3, uint32_t(kNoAllocMaxBlocks));
+  const uint32_t blocks = std::min(uint32_t(sms) * 4, uint32_t(kNoAllocMaxBlocks));
   sq::PauliTilePlan P;  // 26 KiB on the stack
   if (sq::plan_pauli_tiles(P, n, idx, n_terms, 0, xm, zym, ny, weights, blocks) != n_terms)
     return fail(SQ_ERR_UNSUPPORTED, "sq_expect_pauli_noalloc: the terms do not fit one plan");

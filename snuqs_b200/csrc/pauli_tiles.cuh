@@ -4,19 +4,19 @@
 // What bounds it: one read of the state per pass, against one shared-memory
 // read and three FP64 operations per pair and group.  A block holds one tile
 // of 2^11 amplitudes (32 KiB as complex doubles) and each of its 256 threads
-// the eight amplitudes r * 256 + tid of it in registers; a pair's partner is
-// then one 16-byte shared read (lanes read an XOR of consecutive slots:
-// conflict-free without a swizzle), and each pair is taken by one thread:
-//  - the flip reaches register bits: the threads take the four of their
-//    amplitudes with the lowest flipped register bit clear;
-//  - else the thread with the highest flipped thread bit clear takes
-//    amplitudes 0..3, its partner 4..7 (the term is symmetric in the pair).
-// Signs (-1)^popc(i & zy) split over tile base, thread and register: the
-// base's parities are computed once per tile and term, the rows' by the host.
-// Measured on B200, 25 qubits complex128: 64 random strings (8 passes) and 25
-// diagonal ones 2110 us together, before with one read of the state per mask
-// 6212 us; the energy pass of 512 VQE circuits of 8..20 qubits 5.9 ms, before
-// 11.9 ms.
+// four of its amplitudes (r * 256 + tid, rows r = 0..3) in registers.  A group whose flip
+// reaches the top tile bit (the plan makes nearly all do) has one amplitude
+// of every pair in rows 0..3: four partners per thread, each one 16-byte
+// shared read (lanes read an XOR of consecutive slots: conflict-free without
+// a swizzle).  Signs (-1)^popc(i & zy) split over tile base, thread and row:
+// the base's parities are computed once per tile and term, the rows' are two
+// factors of +-1 that the sum over the rows takes in its FMAs.
+// Bound by shared-memory reads (ncu: 80 % of their rate, DRAM 42 %).  Measured
+// on B200: 64 random strings (8 passes) and 25 diagonal ones on 25 qubits
+// complex128 1187 us together, with one read of the state per mask 6212 us;
+// 2110 us with per-row sign flips and own amplitudes chosen at run time, 1670
+// us with a group header and a term loop for every single string.  The energy
+// pass of 512 VQE circuits of 8..20 qubits: 4.0 ms, before 11.9 ms.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -33,73 +33,121 @@ __device__ __forceinline__ double pauli_signed(double v, uint32_t bit31) {
   return __hiloint2double(__double2hiint(v) ^ int(bit31 & 0x80000000u), __double2loint(v));
 }
 
+struct alignas(16) PauliTerm {
+  double f;
+  uint32_t word;  // Z-or-Y mask in tile coordinates | parity of the tile base << 31
+  uint32_t c;     // flip mask of its group
+};
 struct PauliShared {
   double2 *tile;
+  PauliTerm *term;
+  double2 *sign;  // per term: +-1 for row bits 0 and 1
   PauliTileGroup *group;
-  double *f;
-  uint32_t *word;  // thread bits of the Z-or-Y mask | row parities << 16 | parity of the tile base << 31
-  __device__ PauliShared(unsigned char *raw, uint32_t terms, uint32_t groups) {
+  __device__ PauliShared(unsigned char *raw, uint32_t terms) {
     tile = reinterpret_cast<double2 *>(raw);
-    group = reinterpret_cast<PauliTileGroup *>(raw + (16u << kPauliTileBits));
-    f = reinterpret_cast<double *>(group + groups);
-    word = reinterpret_cast<uint32_t *>(f + terms);
+    term = reinterpret_cast<PauliTerm *>(tile + (1u << kPauliTileBits));
+    sign = reinterpret_cast<double2 *>(term + terms);
+    group = reinterpret_cast<PauliTileGroup *>(sign + terms);
   }
 };
 
-// Thread's share of one group.  PB: register bit the four amplitudes have
-// clear; PB < 0: no register bit is flipped (half = the thread's pivot bit).
-template <int PB, bool FULL>
-__device__ __forceinline__ double pauli_group(const double2 (&A)[kPauliRows], const PauliShared &S,
-                                              const PauliTileGroup &G, uint32_t tb, uint32_t rows, uint32_t half) {
-  const uint32_t tid = threadIdx.x, c = G.c;
-  const double2 *partner = S.tile + (tid ^ (c & (kPauliThreads - 1)));
-  const uint32_t cr = c / kPauliThreads;
-  double q[4];
-  uint32_t row[4];
+// Pair product of one group: Re conj(a) b, or Im conj(a) b for an odd number
+// of Y (either amplitude of the pair may be a: the signs make up for it).
+template <bool ODD>
+__device__ __forceinline__ double pauli_pair(const double2 &a, const double2 &b) {
+  return ODD ? fma(a.x, b.y, -a.y * b.x) : fma(a.x, b.x, a.y * b.y);
+}
+
+// Pair products of the thread's four amplitudes in rows 0..3 under a flip
+// that reaches the top tile bit.
+template <bool ODD>
+__device__ __forceinline__ void pauli_pairs_top(const double2 (&A)[4], const PauliShared &S, uint32_t c,
+                                                double (&q)[4]) {
+  const uint32_t at = threadIdx.x ^ c;
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    double2 a;
-    if constexpr (PB < 0) {
-      row[i] = i + 4 * half;
-      a.x = half ? A[i + 4].x : A[i].x;
-      a.y = half ? A[i + 4].y : A[i].y;
-    } else {
-      constexpr int P = PB < 0 ? 0 : PB;
-      const int r = ((i >> P) << (P + 1)) | (i & ((1 << P) - 1));
-      row[i] = r;
-      a = A[r];
-    }
-    const double2 b = partner[(row[i] ^ cr) * kPauliThreads];
-    q[i] = G.odd ? fma(a.x, b.y, -a.y * b.x) : fma(a.x, b.x, a.y * b.y);
+  for (int i = 0; i < 4; ++i) q[i] = pauli_pair<ODD>(A[i], S.tile[at ^ (i * kPauliThreads)]);
+}
+
+// acc + one term's share of such a group.
+__device__ __forceinline__ double pauli_term_top(const PauliShared &S, const PauliTerm &T, uint32_t t,
+                                                 const double (&q)[4], double acc) {
+  const double2 g = S.sign[t];
+  const double x = fma(g.y, fma(g.x, q[3], q[2]), fma(g.x, q[1], q[0]));
+  return fma(pauli_signed(T.f, uint32_t(__popc(T.word & (threadIdx.x | 0x80000000u))) << 31), x, acc);
+}
+
+// The single-term groups [t0, t1) of a pass (terms in group order).
+template <bool ODD>
+__device__ __forceinline__ double pauli_singles(const double2 (&A)[4], const PauliShared &S, uint32_t t0, uint32_t t1,
+                                                double acc) {
+#pragma unroll 2
+  for (uint32_t t = t0; t < t1; ++t) {
+    const PauliTerm T = S.term[t];
+    double q[4];
+    pauli_pairs_top<ODD>(A, S, T.c, q);
+    acc = pauli_term_top(S, T, t, q, acc);
   }
+  return acc;
+}
+
+template <bool ODD>
+__device__ __forceinline__ double pauli_group_top(const double2 (&A)[4], const PauliShared &S,
+                                                  const PauliTileGroup &G, double acc) {
+  double q[4];
+  pauli_pairs_top<ODD>(A, S, G.c, q);
+  for (uint32_t t = G.t0; t < G.t1; ++t) acc = pauli_term_top(S, S.term[t], t, q, acc);
+  return acc;
+}
+
+// Any other off-diagonal group, on a tile of 2^m amplitudes: pairs are
+// numbered by inserting a zero at the highest flipped bit.
+__device__ __forceinline__ double pauli_group_any(const PauliShared &S, const PauliTileGroup &G, uint32_t m) {
+  const uint32_t pivot = 31 - __clz(int(G.c));
   double s = 0.0;
-  for (uint32_t t = G.t0; t < G.t1; ++t) {
-    const uint32_t word = S.word[t], sg = uint32_t(__popc(word & tb)) << 31;
-    double x = 0.0;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const double v = pauli_signed(q[i], sg ^ (word << (15 - row[i])));
-      if (FULL || row[i] < rows) x += v;
-    }
-    s = fma(S.f[t], x, s);
+  for (uint32_t i = 0; i < 4; ++i) {
+    const uint32_t k = i * kPauliThreads + threadIdx.x;
+    if (k >> (m - 1)) break;
+    const uint32_t j = uint32_t(insert_zero(k, pivot));
+    const double2 a = S.tile[j], b = S.tile[j ^ G.c];
+    const double q = G.odd ? pauli_pair<true>(a, b) : pauli_pair<false>(a, b);
+    double w = 0.0;
+    for (uint32_t t = G.t0; t < G.t1; ++t)
+      w += pauli_signed(S.term[t].f, uint32_t(__popc(S.term[t].word & (j | 0x80000000u))) << 31);
+    s = fma(q, w, s);
   }
   return s;
 }
 
-template <bool FULL>
-__device__ __forceinline__ double pauli_diagonal(const double2 (&A)[kPauliRows], const PauliShared &S,
-                                                 const PauliTileGroup &G, uint32_t tb, uint32_t rows) {
-  double w[kPauliRows] = {};
-  for (uint32_t t = G.t0; t < G.t1; ++t) {
-    const uint32_t word = S.word[t];
-    const double f = pauli_signed(S.f[t], uint32_t(__popc(word & tb)) << 31);
+// The diagonal group: the eight rows' probabilities under the eight sign
+// patterns of the row bits (a Walsh transform), then one weight per pattern.
+__device__ __forceinline__ double pauli_diagonal(const PauliShared &S, const PauliTileGroup &G,
+                                                 const uint16_t *diag) {
+  double p[kPauliRows];
 #pragma unroll
-    for (int r = 0; r < kPauliRows; ++r) w[r] += pauli_signed(f, word << (15 - r));
+  for (int r = 0; r < kPauliRows; ++r) {
+    const double2 a = S.tile[r * kPauliThreads + threadIdx.x];
+    p[r] = fma(a.x, a.x, a.y * a.y);
   }
+#pragma unroll
+  for (int b = 1; b < kPauliRows; b <<= 1)
+#pragma unroll
+    for (int r = 0; r < kPauliRows; ++r)
+      if (!(r & b)) {
+        const double u = p[r], v = p[r | b];
+        p[r] = u + v;
+        p[r | b] = u - v;
+      }
+  const uint32_t tb = threadIdx.x | 0x80000000u;
   double s = 0.0;
 #pragma unroll
-  for (int r = 0; r < kPauliRows; ++r)
-    if (FULL || uint32_t(r) < rows) s = fma(fma(A[r].x, A[r].x, A[r].y * A[r].y), w[r], s);
+  for (int z = 0; z < kPauliRows; ++z) {
+    if (diag[z] == diag[z + 1]) continue;
+    double w = 0.0;
+    for (uint32_t t = G.t0 + diag[z]; t < uint32_t(G.t0 + diag[z + 1]); ++t)
+      w += pauli_signed(S.term[t].f, uint32_t(__popc(S.term[t].word & tb)) << 31);
+    s = fma(p[z], w, s);
+  }
   return s;
 }
 
@@ -107,7 +155,13 @@ __device__ __forceinline__ double pauli_diagonal(const double2 (&A)[kPauliRows],
 // Ends without a barrier.
 __device__ __forceinline__ void pauli_stage(const PauliTilePlan &T, const PauliTilePass &S, PauliShared &sh) {
   const uint32_t t0 = T.group[S.g0].t0, t1 = T.group[S.g1 - 1].t1;
-  for (uint32_t i = threadIdx.x; i < t1 - t0; i += kPauliThreads) sh.f[i] = T.f[t0 + i];
+  const uint32_t singles = uint32_t(S.go - S.g0);  // their terms come first
+  for (uint32_t i = threadIdx.x; i < t1 - t0; i += kPauliThreads) {
+    const uint32_t z = T.zt[t0 + i];
+    sh.term[i].f = T.f[t0 + i];
+    sh.term[i].c = i < singles ? T.group[S.g0 + i].c : 0u;
+    sh.sign[i] = make_double2(z & 256u ? -1.0 : 1.0, z & 512u ? -1.0 : 1.0);
+  }
   for (uint32_t i = threadIdx.x; i < uint32_t(S.g1 - S.g0); i += kPauliThreads) {
     PauliTileGroup g = T.group[S.g0 + i];
     g.t0 = uint16_t(g.t0 - t0);
@@ -128,7 +182,7 @@ __device__ __forceinline__ double pauli_tile(const typename Vec2<Real>::T *__res
   for (uint32_t i = low; i < 8 && i < m; ++i)
     if ((tid >> i) & 1) mine ^= S.gen[i - low];
   const uint32_t rows = FULL ? kPauliRows : (m > 8 ? 1u << (m - 8) : (tid >> m) == 0 ? 1u : 0u);
-  double2 A[kPauliRows];
+  double2 A[4];
   {
     typename Vec2<Real>::T v[kPauliRows];
 #pragma unroll
@@ -145,38 +199,27 @@ __device__ __forceinline__ double pauli_tile(const typename Vec2<Real>::T *__res
       }
     }
 #pragma unroll
-    for (int r = 0; r < kPauliRows; ++r) A[r] = make_double2(double(v[r].x), double(v[r].y));
+    for (int r = 0; r < kPauliRows; ++r) {
+      const double2 a = make_double2(double(v[r].x), double(v[r].y));
+      if (r < 4) A[r] = a;
+      sh.tile[r * kPauliThreads + tid] = a;
+    }
   }
-#pragma unroll
-  for (int r = 0; r < kPauliRows; ++r) sh.tile[r * kPauliThreads + tid] = A[r];
   const uint32_t t0 = T.group[S.g0].t0, t1 = T.group[S.g1 - 1].t1;
   for (uint32_t i = tid; i < t1 - t0; i += kPauliThreads)
-    sh.word[i] = (T.zt[t0 + i] & 0xff00ffu) | (uint32_t(__popcll(base & T.zy[t0 + i])) << 31);
+    sh.term[i].word = T.zt[t0 + i] | (uint32_t(__popcll(base & T.zy[t0 + i])) << 31);
   __syncthreads();
-  const uint32_t tb = tid | 0x80000000u;
-  double acc = 0.0;
-  for (uint32_t g = 0; g < uint32_t(S.g1 - S.g0); ++g) {
+  const uint32_t even = uint32_t(S.ge - S.g0), odd = uint32_t(S.go - S.g0);
+  double acc = pauli_singles<false>(A, sh, 0, even, 0.0);
+  acc = pauli_singles<true>(A, sh, even, odd, acc);
+  for (uint32_t g = odd; g < uint32_t(S.g1 - S.g0); ++g) {
     const PauliTileGroup G = sh.group[g];
-    const uint32_t cr = G.c / kPauliThreads;
-    if (G.c == 0) {
-      acc += pauli_diagonal<FULL>(A, sh, G, tb, rows);
-    } else if (cr & 1) {
-      acc += pauli_group<0, FULL>(A, sh, G, tb, rows, 0);
-    } else if (cr & 2) {
-      acc += pauli_group<1, FULL>(A, sh, G, tb, rows, 0);
-    } else if (cr) {
-      acc += pauli_group<2, FULL>(A, sh, G, tb, rows, 0);
-    } else {
-      const uint32_t half = (tid >> (31 - __clz(int(G.c)))) & 1u;
-      if (FULL) {
-        acc += pauli_group<-1, FULL>(A, sh, G, tb, rows, half);
-      } else {
-        // Fewer than eight rows: the thread with the pivot bit clear takes
-        // all of its amplitudes (rows 4..7 do not exist below 2^11).
-        const double s = pauli_group<-1, FULL>(A, sh, G, tb, rows, 0);
-        acc += half ? 0.0 : s;
-      }
-    }
+    if (FULL && (G.c >> (kPauliTileBits - 1)))
+      acc = G.odd ? pauli_group_top<true>(A, sh, G, acc) : pauli_group_top<false>(A, sh, G, acc);
+    else if (G.c)
+      acc += pauli_group_any(sh, G, m);
+    else if (FULL || rows)
+      acc += pauli_diagonal(sh, G, T.diag);
   }
   __syncthreads();
   return acc;
@@ -184,11 +227,11 @@ __device__ __forceinline__ double pauli_tile(const typename Vec2<Real>::T *__res
 
 // partial[blockIdx.x] (+)= this block's share of the plan's expectation.
 template <typename Real, bool FULL>
-__global__ void __launch_bounds__(kPauliThreads, 3)
+__global__ void __launch_bounds__(kPauliThreads, 4)
     pauli_expect_tiles(const typename Vec2<Real>::T *__restrict__ psi, const __grid_constant__ PauliTilePlan T,
                        double *__restrict__ partial, int accumulate) {
   extern __shared__ __align__(16) unsigned char pauli_raw[];
-  PauliShared sh(pauli_raw, T.max_terms, T.max_groups);
+  PauliShared sh(pauli_raw, T.max_terms);
   const uint32_t tile_bits = T.n - T.m;
   const uint64_t items = uint64_t(T.npasses) << tile_bits;
   uint32_t staged = ~0u;

@@ -11,6 +11,13 @@
 // runs of complex128 amplitudes, and eight more generators), and the state is
 // read once per pass: 64 random strings of 25 qubits take 8 passes instead
 // of 64 reads.
+//
+// The span's basis is chosen so that the top tile bit is set in the tile
+// coordinates of every mask that made the span grow (a linear functional l
+// with l(mask) = 1: possible because those masks are independent).  Both
+// amplitudes of such a pair then lie in different halves of the tile, at
+// places the kernel knows at compile time; a mask inside the span with l = 0
+// takes the kernel's slower general form.
 #pragma once
 #include <stdint.h>
 
@@ -32,7 +39,9 @@ struct alignas(8) PauliTileGroup {
 struct PauliTilePass {
   uint64_t gen[kPauliGens];    // global index vector of tile bit low + i
   uint8_t pivot[kPauliGens];   // ascending bits the tile base has clear
-  uint16_t g0, g1;             // groups
+  // Groups: single terms that flip the top tile bit with an even number of Y
+  // [g0, ge) and an odd one [ge, go), all others [go, g1).
+  uint16_t g0, ge, go, g1;
 };
 
 // Tile index j stands for global index base ^ (j's low bits) ^ gens of its
@@ -46,15 +55,16 @@ struct PauliTilePlan {
   PauliTileGroup group[kPauliMaxGroups];
   uint64_t zy[kPauliMaxTerms];   // Z-or-Y mask (global index bits)
   double f[kPauliMaxTerms];      // weight and phase
-  // Z-or-Y mask in tile coordinates (bits 0..10), and at bit 16 + r its parity
-  // on tile row r (tile bits 8 and up).
-  uint32_t zt[kPauliMaxTerms];
+  uint32_t zt[kPauliMaxTerms];   // Z-or-Y mask in tile coordinates
+  // Terms of the diagonal group (at most one), relative to its first: those
+  // with row parities z (tile bits 8..10 of zt) are diag[z] .. diag[z + 1].
+  uint16_t diag[9];
 };
 
 // Dynamic shared memory of the kernels for passes of at most these sizes:
-// the tile as complex doubles, the groups, per term a weight and a word.
+// the tile as complex doubles, two 16-byte records per term, the groups.
 constexpr uint32_t pauli_tile_smem(uint32_t terms, uint32_t groups) {
-  return (16u << kPauliTileBits) + groups * 8u + terms * 12u;
+  return (16u << kPauliTileBits) + groups * 8u + terms * 32u;
 }
 
 // Plans the groups that start at term position `pos` of the term order idx
@@ -102,73 +112,116 @@ uint32_t plan_pauli_tiles(PauliTilePlan &P, uint32_t n, const Index *idx, uint32
     PauliTilePass &S = P.pass[P.npasses++];
     uint64_t gen[kPauliGens];
     uint32_t piv[kPauliGens], dim = 0;
-    // gen stays reduced: bit piv[i] is set in gen[i] only.
-    auto add = [&](uint64_t x) -> bool {
+    bool val[kPauliGens];  // l(gen[i])
+    // gen stays reduced: bit piv[i] is set in gen[i] only.  Adds x with l(x) = v.
+    auto add = [&](uint64_t x, bool v) -> bool {
       for (uint32_t i = 0; i < dim; ++i)
-        if ((x >> piv[i]) & 1) x ^= gen[i];
+        if ((x >> piv[i]) & 1) {
+          x ^= gen[i];
+          v ^= val[i];
+        }
       if (!x) return true;
       if (dim == gens) return false;
       uint32_t p = 0;
       while (!((x >> p) & 1)) ++p;
       for (uint32_t i = 0; i < dim; ++i)
-        if ((gen[i] >> p) & 1) gen[i] ^= x;
+        if ((gen[i] >> p) & 1) {
+          gen[i] ^= x;
+          val[i] ^= v;
+        }
       gen[dim] = x;
+      val[dim] = v;
       piv[dim++] = p;
       return true;
     };
     uint16_t member[kPauliMaxGroups];
     uint32_t nm = 0;
     for (uint32_t g = 0; g < ngroups && nm < cap; ++g)
-      if (!taken[g] && add(xm[idx[base + first[g]]] & ~lowmask)) {
+      if (!taken[g] && add(xm[idx[base + first[g]]] & ~lowmask, true)) {
         taken[g] = true;
         member[nm++] = uint16_t(g);
       }
     left -= nm;
-    for (uint32_t b = P.low; dim < gens; ++b) add(uint64_t(1) << b);  // fill with the lowest free bits
-    // Tile bits in ascending pivot order.
+    for (uint32_t b = P.low; dim < gens; ++b) add(uint64_t(1) << b, false);  // fill with the lowest free bits
+    // The top tile bit: a generator with l = 1, which the others with l = 1
+    // then lose; the rest in ascending pivot order.
+    auto exchange = [&](uint32_t i, uint32_t j) {
+      const uint32_t tp = piv[i];
+      piv[i] = piv[j];
+      piv[j] = tp;
+      const uint64_t tg = gen[i];
+      gen[i] = gen[j];
+      gen[j] = tg;
+      const bool tv = val[i];
+      val[i] = val[j];
+      val[j] = tv;
+    };
     for (uint32_t i = 0; i < gens; ++i)
-      for (uint32_t j = i + 1; j < gens; ++j)
-        if (piv[j] < piv[i]) {
-          const uint32_t tp = piv[i];
-          piv[i] = piv[j];
-          piv[j] = tp;
-          const uint64_t tg = gen[i];
-          gen[i] = gen[j];
-          gen[j] = tg;
-        }
-    for (uint32_t i = 0; i < kPauliGens; ++i) {
+      if (val[i]) {
+        exchange(i, gens - 1);
+        for (uint32_t j = 0; j + 1 < gens; ++j)
+          if (val[j]) gen[j] ^= gen[gens - 1];
+        break;
+      }
+    for (uint32_t i = 0; i + 1 < gens; ++i)
+      for (uint32_t j = i + 1; j + 1 < gens; ++j)
+        if (piv[j] < piv[i]) exchange(i, j);
+    // The tile base has the pivots clear: ascending for its enumeration.
+    uint64_t pivots = 0;
+    for (uint32_t i = 0; i < gens; ++i) pivots |= uint64_t(1) << piv[i];
+    for (uint32_t i = 0, p = 0; i < kPauliGens; ++i) {
       S.gen[i] = i < gens ? gen[i] : 0;
-      S.pivot[i] = uint8_t(i < gens ? piv[i] : 0);
+      while (pivots >> p && !((pivots >> p) & 1)) ++p;
+      S.pivot[i] = uint8_t(i < gens ? p++ : 0);
     }
     S.g0 = uint16_t(ng);
     const uint32_t t_begin = nt;
-    for (uint32_t k = 0; k < nm; ++k) {
-      const uint32_t g = member[k], i0 = idx[base + first[g]];
-      const uint64_t x = xm[i0];
-      PauliTileGroup &G = P.group[ng++];
+    auto coordinate_of = [&](uint64_t x) {
+      // Every pivot but the top generator's occurs in one generator only;
+      // what is left then tells the top one's.
       uint64_t rest = x;
       uint32_t c = 0;
       for (uint32_t i = 0; i < gens; ++i)
-        if ((x >> piv[i]) & 1) {
+        if (((i + 1 < gens ? x : rest) >> piv[i]) & 1) {
           c |= 1u << (P.low + i);
           rest ^= gen[i];
         }
-      G.c = uint16_t(c | uint32_t(rest));
+      return c | uint32_t(rest);
+    };
+    for (uint32_t k = 0; k < 3 * nm; ++k) {
+      if (k == nm) S.ge = uint16_t(ng);
+      if (k == 2 * nm) S.go = uint16_t(ng);
+      const uint32_t g = member[k % nm], i0 = idx[base + first[g]];
+      const uint64_t x = xm[i0];
+      const uint32_t c = coordinate_of(x);
+      const bool single = last[g] - first[g] == 1 && (c >> (kPauliTileBits - 1));
+      if ((single ? uint32_t(ny[i0] & 1) : 2u) != k / nm) continue;
+      PauliTileGroup &G = P.group[ng++];
+      G.c = uint16_t(c);
       G.odd = uint16_t(ny[i0] & 1);
       G.t0 = uint16_t(nt);
-      for (uint32_t e = first[g]; e < last[g]; ++e) {
-        const uint32_t t = idx[base + e];
+      auto put = [&](uint32_t t, uint32_t zt) {
         P.zy[nt] = zym[t];
         // (-i)^ny folded into a real factor: even ny (-1)^(ny/2), odd ny
         // (-1)^((ny-1)/2) for the imaginary part; a pair counts twice.
         P.f[nt] = w[t] * (((ny[t] / 2) & 1) ? -1.0 : 1.0) * (x ? 2.0 : 1.0);
+        P.zt[nt++] = zt;
+      };
+      auto coordinates = [&](uint32_t t) {
         uint32_t zt = uint32_t(zym[t] & lowmask);
         for (uint32_t i = 0; i < gens; ++i)
           if (__builtin_popcountll(gen[i] & zym[t]) & 1) zt |= 1u << (P.low + i);
-        for (uint32_t r = 0; r < 8; ++r)
-          if (__builtin_popcount((r << 8) & zt) & 1) zt |= 1u << (16 + r);
-        P.zt[nt++] = zt;
+        return zt;
+      };
+      // The diagonal group's terms by row parities.
+      for (uint32_t z = 0; z < (x ? 1u : 8u); ++z) {
+        if (!x) P.diag[z] = uint16_t(nt - G.t0);
+        for (uint32_t e = first[g]; e < last[g]; ++e) {
+          const uint32_t t = idx[base + e], zt = coordinates(t);
+          if (x || zt >> 8 == z) put(t, zt);
+        }
       }
+      if (!x) P.diag[8] = uint16_t(nt - G.t0);
       G.t1 = uint16_t(nt);
     }
     S.g1 = uint16_t(ng);
