@@ -12,7 +12,9 @@
 #include "adjoint_plan.h"
 
 #include <cstring>
+#include <map>
 #include <stdexcept>
+#include <utility>
 
 namespace sq {
 
@@ -75,6 +77,7 @@ void build_adjoint(const sq_circuit_op *ops, uint32_t nops, uint32_t n, AdjointP
     HostOp h;
     if (analyse_op(m, index_bits(op, n), 0, 0, h)) out.forward.push_back(h);
   }
+  std::map<std::pair<int32_t, double>, uint32_t> slot_of;
   for (uint32_t i = nops; i-- > 0;) {
     const sq_circuit_op &op = ops[i];
     const int d = 1 << op.k;
@@ -102,8 +105,11 @@ void build_adjoint(const sq_circuit_op *ops, uint32_t nops, uint32_t n, AdjointP
         } else {
           ip.m = K;
         }
-        ip.slot = uint32_t(out.occurrences.size());
-        out.occurrences.push_back({op.param[a], op.scale[a]});
+        // Angles that follow one parameter with one factor share a slot.
+        const auto key = std::make_pair(int32_t(op.param[a]), double(op.scale[a]));
+        const auto it = slot_of.emplace(key, uint32_t(out.occurrences.size()));
+        if (it.second) out.occurrences.push_back(key);
+        ip.slot = it.first->second;
         out.reverse.push_back(ip);
       }
     }

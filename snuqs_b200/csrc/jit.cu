@@ -335,28 +335,62 @@ bool lane_indexed(const SweepOp &op) {
   return false;
 }
 
-// Call of the inner-product routine of a kSwInnerDiag / kSwInnerDense op
-// (`bits`: the statement that sets b, the op's non-register target bits),
-// accumulating into doubles sr, si.  Pauli-form ops (kAuxPauli) take the
-// four-FMA-per-amplitude routines.
-std::string inner_call(const SweepOp &op, const char *R, const std::string &bits) {
+// Inner-product slots a reverse sweep keeps as one double per thread, added up
+// over the thread's tiles and summed over the warp once at the end; further
+// slots are summed over the warp for every tile (ten shuffles).  The sweeps are
+// bound by FP64 issue.  Measured on B200 (QAOA p = 8, 24 qubits complex128):
+// 20 reverse sweeps 5.9 ms with this, the real part alone and the shared sums
+// of the diagonal generators; 10.1 ms with complex inner products, each summed
+// over the warp for every tile.
+constexpr uint32_t kRegSlots = 8;
+
+// Adds `expr` (a thread's share) to slot `slot`.
+std::string inner_add(uint32_t slot, const std::string &expr, int NT) {
   std::ostringstream s;
+  if (slot < kRegSlots)
+    s << "ip" << slot << " += " << expr << ";";
+  else
+    s << "jit_inner_acc<" << NT << ", " << slot << ">(acc, " << expr << ");";
+  return s.str();
+}
+
+// The register slots of a sweep's ops: their declarations, or the code that
+// hands them to the warps' sums after the last tile.
+std::string inner_slots(const SweepOp *ops, size_t nops, bool finish, int NT) {
+  uint32_t n = 0;
+  for (size_t i = 0; i < nops; ++i)
+    if (ops[i].kind == kSwInnerDiag || ops[i].kind == kSwInnerDense) n = std::max(n, ops[i].slot + 1);
+  std::ostringstream s;
+  for (uint32_t i = 0; i < std::min(n, kRegSlots); ++i)
+    if (finish)
+      s << " jit_inner_acc<" << NT << ", " << i << ">(acc, ip" << i << ");";
+    else
+      s << " double ip" << i << " = 0.0;";
+  return s.str();
+}
+
+// Statement adding the real part of a kSwInnerDiag / kSwInnerDense op's inner
+// product to its slot (`bits`: the statement that sets b, the op's
+// non-register target bits).
+std::string inner_call(const SweepOp &op, const char *R, const std::string &bits, int NT) {
+  std::ostringstream s, e;
   const bool pauli = op.aux & kAuxPauli;
-  if (op.kind == kSwInnerDiag) {
-    s << bits << " ";
-    if (pauli)
-      s << "inner_diag_pauli<" << R << ", " << int(op.vmask) << ", " << int(op.aux & 7) << ">";
-    else
-      s << "inner_diag<" << R << ", " << int(op.vmask) << ">";
-    s << "(F, G, coef + " << op.coef << ", b, sr, si); ";
+  if (op.kind == kSwInnerDiag) s << bits << " ";
+  if (pauli && op.kind == kSwInnerDiag) {
+    e << "real_inner_diag_pauli<" << R << ", " << int(op.vmask) << ", " << int(op.aux & 7) << ">(F, G, coef + "
+      << op.coef << ", b)";
+  } else if (pauli) {
+    e << "real_inner_dense_pauli<" << R << ", " << int(op.vmask) << ", " << int(op.aux & 7) << ", "
+      << int((op.aux >> 3) & 7) << ">(F, G, coef + " << op.coef << ")";
   } else {
-    if (pauli)
-      s << "inner_dense_pauli<" << R << ", " << int(op.vmask) << ", " << int(op.aux & 7) << ", "
-        << int((op.aux >> 3) & 7) << ">";
+    s << "double sr = 0.0, si = 0.0; ";
+    if (op.kind == kSwInnerDiag)
+      s << "inner_diag<" << R << ", " << int(op.vmask) << ">(F, G, coef + " << op.coef << ", b, sr, si); ";
     else
-      s << "inner_dense<" << R << ", " << int(op.vmask) << ">";
-    s << "(F, G, coef + " << op.coef << ", sr, si); ";
+      s << "inner_dense<" << R << ", " << int(op.vmask) << ">(F, G, coef + " << op.coef << ", sr, si); ";
+    e << "sr";
   }
+  s << inner_add(op.slot, e.str(), NT);
   return s.str();
 }
 
@@ -611,8 +645,7 @@ void one_state_ops_src(const SweepOp *ops, const SweepPhase &ph, const char *R, 
 bool two_state_ops_src(const SweepOp *ops, const SweepPhase &ph, const char *R, bool c64, int NT, std::ostream &s) {
   auto cf = [](const SweepOp &o) { return "(coef + " + std::to_string(o.coef) + ")"; };
   auto inner_plain = [&](const SweepOp &op) {
-    s << "      { double sr = 0.0, si = 0.0; " << inner_call(op, R, diag_bits_src(op)) << "jit_inner_acc<" << NT
-      << ", " << op.slot << ">(acc, sr, si); }\n";
+    s << "      { " << inner_call(op, R, diag_bits_src(op), NT) << " }\n";
   };
   auto single = [&](const SweepOp &op) {
     std::string tmpl;
@@ -651,25 +684,31 @@ bool two_state_ops_src(const SweepOp *ops, const SweepPhase &ph, const char *R, 
         diag.push_back(&op);
     }
     if (!pauli.empty()) {
+      // Im conj(lambda_r) phi_r once per amplitude (alpha is imaginary, so the
+      // gradient needs no more), and its sums under the eight sign patterns
+      // of the register bits by a Walsh transform (24 additions); an op is
+      // then one of them times its sign on the thread's and tile's bits.
       s << "      { // " << pauli.size() << " Pauli-Z inner products from shared products\n";
       for (int ri = 0; ri < kAdjAmps; ++ri)
-        s << "        const double p" << ri << "r = fma(double(G.re[" << ri << "]), double(F.re[" << ri
-          << "]), double(G.im[" << ri << "]) * double(F.im[" << ri << "])), p" << ri << "i = fma(double(G.re["
-          << ri << "]), double(F.im[" << ri << "]), -double(G.im[" << ri << "]) * double(F.re[" << ri << "]));\n";
+        s << "        const double p0_" << ri << " = fma(double(G.re[" << ri << "]), double(F.im[" << ri
+          << "]), -double(G.im[" << ri << "]) * double(F.re[" << ri << "]));\n";
+      for (int b = 0; b < kAdjRegBits; ++b)
+        for (int ri = 0; ri < kAdjAmps; ++ri)
+          s << "        const double p" << b + 1 << "_" << ri << " = p" << b << "_" << (ri & ~(1 << b))
+            << (((ri >> b) & 1) ? " - p" : " + p") << b << "_" << (ri | (1 << b)) << ";\n";
       for (const SweepOp *op : pauli) {
         const int V = op->vmask, Z = op->aux & 7, nv = __builtin_popcount(uint32_t(V));
-        std::ostringstream qr, qi;
-        for (int ri = 0; ri < kAdjAmps; ++ri) {
-          const bool neg = __builtin_popcount(uint32_t(bit_ext(ri, V) & Z)) & 1;
-          qr << (neg ? " - " : " + ") << "p" << ri << "r";
-          qi << (neg ? " - " : " + ") << "p" << ri << "i";
-        }
-        s << "        { double qr = 0.0" << qr.str() << ", qi = 0.0" << qi.str() << ";";
+        const int rz = bit_dep(Z & ((1 << nv) - 1), V);  // sign pattern over the register bits
+        std::ostringstream e;
+        e << "-double((" << cf(*op) << "[0]).y) * ";
         if (Z >> nv)
-          s << " " << diag_bits_src(*op) << " if (__popc(b & " << (Z >> nv) << "u) & 1) { qr = -qr; qi = -qi; }";
-        s << "\n          const auto a = " << cf(*op) << "[0];\n"
-          << "          jit_inner_acc<" << NT << ", " << op->slot << ">(acc, double(a.x) * qr - double(a.y) * qi, "
-          << "double(a.x) * qi + double(a.y) * qr); }\n";
+          e << "((__popc(b & " << (Z >> nv) << "u) & 1) ? -p" << kAdjRegBits << "_" << rz << " : p" << kAdjRegBits
+            << "_" << rz << ")";
+        else
+          e << "p" << kAdjRegBits << "_" << rz;
+        s << "        { ";
+        if (Z >> nv) s << diag_bits_src(*op) << " ";
+        s << inner_add(op->slot, e.str(), NT) << " }\n";
       }
       s << "      }\n";
     }
@@ -881,6 +920,7 @@ std::string jit_adjoint_body(const PlannedSweep &ps, bool c64, int minb) {
   s << "  using Tile = JitTile<" << M << ", " << ps.h.l;
   for (uint32_t i = 0; i < ps.h.m - ps.h.l; ++i) s << ", " << int(ps.h.hi[i]);
   s << ">;\n";
+  s << " " << inner_slots(ps.op.data(), ps.op.size(), false, NT) << "\n";
   s << "  jit_adjoint_sweep<" << R << ", " << M
     << ", Tile>(psi, lam, P, partials, [&](C2 *ft, C2 *lt, const C2 *coef, uint64_t gbase, double2 *acc) {\n";
   for (uint32_t p = 0; p < ps.h.nphases; ++p) {
@@ -895,7 +935,7 @@ std::string jit_adjoint_body(const PlannedSweep &ps, bool c64, int minb) {
     if (!two_state_ops_src(ps.op.data(), ph, R, c64, NT, s)) return std::string();
     s << "      Ph::scatter(F, G, ft, lt, jb);\n      __syncthreads();\n    }\n";
   }
-  s << "  });\n}\n";
+  s << "  }, [&](double2 *acc) {" << inner_slots(ps.op.data(), ps.op.size(), true, NT) << " });\n}\n";
   return s.str();
 }
 
@@ -951,7 +991,7 @@ std::string jit_batch_adjoint_body(const unsigned char *plan, uint32_t nfwd, uin
       fns << "  jit_batch_fwd<" << R << ", " << M << ", Tile>(psi, bufs, " << ps.h.num_tiles
           << "ull, [&](C2 *tile, uint64_t gbase) {\n";
     else
-      fns << "  jit_batch_rev<" << R << ", " << M << ", Tile>(psi, lam, bufs, " << ps.h.num_tiles
+      fns << " " << inner_slots(ops, ps.nops, false, NT) << "\n  jit_batch_rev<" << R << ", " << M << ", Tile>(psi, lam, bufs, " << ps.h.num_tiles
           << "ull, [&](C2 *ft, C2 *lt, uint64_t gbase) {\n";
     for (uint32_t p = 0; p < ps.h.nphases; ++p) {
       const SweepPhase &P = ph[p];
@@ -978,6 +1018,7 @@ std::string jit_batch_adjoint_body(const unsigned char *plan, uint32_t nfwd, uin
       }
     }
     fns << "  });\n";
+    if (rev) fns << " " << inner_slots(ops, ps.nops, true, NT) << "\n  __syncthreads();\n";
     if (rev && inner) {
       fns << "  if (threadIdx.x == 0) {\n";
       for (uint32_t q = 0; q < inner[0]; ++q)

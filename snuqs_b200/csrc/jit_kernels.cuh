@@ -688,21 +688,54 @@ struct JitPhase2 {
   }
 };
 
-// Adds one thread's inner-product share to its warp's slot (warp shuffle,
-// then lane 0 adds to acc[warp * kMaxInner + SLOT]).
+// Real part of one thread's inner product for an op flagged kAuxPauli (the
+// gradient is 2 Re <lambda|K|phi>).  K = alpha P is anti-Hermitian, so alpha is
+// imaginary, or real when P = X^x Z^z is anti-Hermitian (popc(x & z) odd): one
+// of the two parts of the product is needed, two FMAs per amplitude.
+template <typename Real, int V, int X, int Z>
+__device__ __forceinline__ double real_inner_dense_pauli(const Amps<Real, kAdjAmps> &F, const Amps<Real, kAdjAmps> &G,
+                                                         const typename Vec2<Real>::T *__restrict__ c) {
+  constexpr int D = 1 << ct_popc<V>();
+  constexpr bool ANTI = ct_popc<(X & Z)>() & 1;
+  double p = 0.0, m = 0.0;
+#pragma unroll
+  for (int g = 0; g < kAdjAmps; ++g) {
+    if (g & V) continue;
+#pragma unroll
+    for (int r = 0; r < D; ++r) {
+      const int ir = g | ct_dep<V>(r), ix = g | ct_dep<V>(r ^ X);
+      const double gr = double(G.re[ir]), gi = double(G.im[ir]);
+      const double fr = double(F.re[ix]), fi = double(F.im[ix]);
+      double &s = (__popc(uint32_t(r & Z)) & 1) ? m : p;
+      s = ANTI ? fma(gr, fr, fma(gi, fi, s)) : fma(gr, fi, fma(-gi, fr, s));
+    }
+  }
+  const auto a = c[X];
+  return ANTI ? double(a.x) * (p - m) : double(a.y) * (m - p);
+}
+
+// Diagonal form: alpha is imaginary; b: the op's non-register target bits.
+template <typename Real, int V, int Z>
+__device__ __forceinline__ double real_inner_diag_pauli(const Amps<Real, kAdjAmps> &F, const Amps<Real, kAdjAmps> &G,
+                                                        const typename Vec2<Real>::T *__restrict__ c, uint32_t b) {
+  double p = 0.0, m = 0.0;
+#pragma unroll
+  for (int ri = 0; ri < kAdjAmps; ++ri) {
+    double &s = (__popc(uint32_t(ct_ext<V>(ri) & Z)) & 1) ? m : p;
+    s = fma(double(G.re[ri]), double(F.im[ri]), fma(-double(G.im[ri]), double(F.re[ri]), s));
+  }
+  const double q = (__popc(b & uint32_t(Z >> ct_popc<V>())) & 1) ? p - m : m - p;
+  return double(c[0].y) * q;
+}
+
+// Adds one thread's share of slot SLOT to its warp's sum (warp shuffles, then
+// lane 0 adds to acc[warp * kMaxInner + SLOT]).
 template <int NT, int SLOT>
-__device__ __forceinline__ void jit_inner_acc(double2 *acc, double sr, double si) {
+__device__ __forceinline__ void jit_inner_acc(double2 *acc, double s) {
   constexpr unsigned kMask = NT >= 32 ? 0xffffffffu : ((1u << NT) - 1u);
 #pragma unroll
-  for (int off = (NT >= 32 ? 16 : NT / 2); off > 0; off >>= 1) {
-    sr += __shfl_xor_sync(kMask, sr, off);
-    si += __shfl_xor_sync(kMask, si, off);
-  }
-  if ((threadIdx.x & 31) == 0) {
-    double2 &a = acc[(threadIdx.x >> 5) * kMaxInner + SLOT];
-    a.x += sr;
-    a.y += si;
-  }
+  for (int off = (NT >= 32 ? 16 : NT / 2); off > 0; off >>= 1) s += __shfl_xor_sync(kMask, s, off);
+  if ((threadIdx.x & 31) == 0) acc[(threadIdx.x >> 5) * kMaxInner + SLOT].x += s;
 }
 
 // Dynamic shared memory of a JIT adjoint sweep: phi tiles (2 buffers) |
@@ -716,11 +749,12 @@ __host__ __device__ constexpr size_t jit_adjoint_smem_bytes(int m, size_t amp_by
 // phases(ft, lt, coef, gbase, acc) runs every phase of one tile pair.
 // partials[(block * warps + warp) * kMaxInner + slot] receives each warp's
 // sums at the end (as adjoint_sweep_kernel).
-template <typename Real, int M, class Tile, class Phases>
+// finish(acc) runs once after the last tile (per-thread sums to the warp's slots).
+template <typename Real, int M, class Tile, class Phases, class Finish>
 __device__ __forceinline__ void jit_adjoint_sweep(typename Vec2<Real>::T *__restrict__ psi,
                                                   typename Vec2<Real>::T *__restrict__ lam,
                                                   const SweepParams<Real> &P, double2 *__restrict__ partials,
-                                                  Phases phases) {
+                                                  Phases phases, Finish finish) {
   using C2 = typename Vec2<Real>::T;
   constexpr int NT = 1 << (M - kAdjRegBits);
   constexpr int NW = (NT + 31) / 32;
@@ -783,6 +817,7 @@ __device__ __forceinline__ void jit_adjoint_sweep(typename Vec2<Real>::T *__rest
   }
   cp_async_wait_prev();
   asm volatile("cp.async.wait_all;\n" ::: "memory");
+  finish(acc);
   __syncthreads();
   for (uint32_t i = tid; i < NW * kMaxInner; i += NT)
     partials[size_t(blockIdx.x) * NW * kMaxInner + i] = acc[i];

@@ -23,13 +23,28 @@ namespace {
 
 int popc64(uint64_t x) { return __builtin_popcountll(x); }
 
+// The distinct inner-product slots of a sweep (at most kMaxInner).
+struct InnerSlotSet {
+  uint32_t slot[kMaxInner], count = 0;
+  bool has(uint32_t s) const {
+    for (uint32_t i = 0; i < count; ++i)
+      if (slot[i] == s) return true;
+    return false;
+  }
+  bool fits(uint32_t s) const { return count < uint32_t(kMaxInner) || has(s); }
+  void add(uint32_t s) {
+    if (!has(s)) slot[count++] = s;
+  }
+};
+
 struct SweepBuilder {
   uint32_t n, m, l, max_dense_k = 3, reg_bits = kRegBits, max_ops = kMaxOps;
   uint64_t S;  // tile bits (global index bits)
   std::vector<const HostOp *> ops;
   std::vector<uint64_t> phase_regs;  // register bits (global) of each phase
   std::vector<uint32_t> phase_first; // first op index of each phase
-  uint32_t ncoef = 0, ninner = 0;
+  uint32_t ncoef = 0;
+  InnerSlotSet inner;
   // Remap: output global bit of the content of every global bit (size n;
   // empty = the identity).  Only tile bits move.
   std::vector<int> outmap;
@@ -49,7 +64,7 @@ struct SweepBuilder {
   bool try_add(const HostOp &op) {
     if (ops.size() >= size_t(max_ops)) return false;
     if (ncoef + coef_count(op) > uint32_t(kMaxCoef)) return false;
-    if (op.kind == kOpInner && ninner >= uint32_t(kMaxInner)) return false;
+    if (op.kind == kOpInner && !inner.fits(op.slot)) return false;
     if (is_diag(op)) {
       if (op.tbits.size() > size_t(kMaxDiagK)) return false;
       if (phase_regs.empty()) {
@@ -58,7 +73,7 @@ struct SweepBuilder {
       }
       ops.push_back(&op);
       ncoef += coef_count(op);
-      if (op.kind == kOpInner) ++ninner;
+      if (op.kind == kOpInner) inner.add(op.slot);
       return true;
     }
     const uint32_t kmax = op.kind == kOpInner ? reg_bits : max_dense_k;
@@ -76,7 +91,7 @@ struct SweepBuilder {
     }
     ops.push_back(&op);
     ncoef += coef_count(op);
-    if (op.kind == kOpInner) ++ninner;
+    if (op.kind == kOpInner) inner.add(op.slot);
     return true;
   }
 
@@ -108,7 +123,11 @@ bool pauli_form(const cplx *K, int d, bool diag, uint32_t &x, uint32_t &z) {
       const cplx want = c == (r ^ int(x)) ? ((__builtin_popcount(uint32_t(r) & z) & 1) ? -a : a) : cplx(0, 0);
       if (std::abs(at(r, c) - want) > tol) return false;
     }
-  return true;
+  // K = (dU/da) U^dagger is anti-Hermitian for a unitary U, so alpha is
+  // imaginary, or real when P = X^x Z^z is itself anti-Hermitian; the JIT
+  // kernels take that part only.
+  const bool anti = __builtin_popcount(x & z) & 1;
+  return std::abs(anti ? a.imag() : a.real()) <= tol;
 }
 
 // Picks the cheapest sweep-op kind for a dense k-qubit matrix in canonical
@@ -177,6 +196,13 @@ void encode_dense(SweepOp &so, const std::vector<cplx> &cm, int k, std::vector<c
 
 PlannedSweep SweepBuilder::finish() const {
   PlannedSweep ps;
+  // Ops of one global slot share a local one.
+  auto local_slot = [&](uint32_t global) {
+    for (size_t i = 0; i < ps.inner_global.size(); ++i)
+      if (ps.inner_global[i] == global) return uint32_t(i);
+    ps.inner_global.push_back(global);
+    return uint32_t(ps.inner_global.size() - 1);
+  };
   // Pad the tile to exactly m bits with the lowest unused bits.
   uint64_t tile = S;
   for (uint32_t b = 0; b < n && uint32_t(popc64(tile)) < m; ++b) tile |= uint64_t(1) << b;
@@ -276,8 +302,7 @@ PlannedSweep SweepBuilder::finish() const {
         } else {
           so.kind = op.kind == kOpInner ? kSwInnerDiag : kSwDiag;
           if (op.kind == kOpInner) {
-            so.slot = uint32_t(ps.inner_global.size());
-            ps.inner_global.push_back(op.slot);
+            so.slot = local_slot(op.slot);
           }
           // Register targets -> canonical low index bits; the rest -> high
           // bits, most significant first.
@@ -344,8 +369,7 @@ PlannedSweep SweepBuilder::finish() const {
           if ((op.cmask >> b) & 1) add_cond(so, b, (op.cval >> b) & 1);
         if (op.kind == kOpInner) {
           so.kind = kSwInnerDense;
-          so.slot = uint32_t(ps.inner_global.size());
-          ps.inner_global.push_back(op.slot);
+          so.slot = local_slot(op.slot);
           uint32_t px = 0, pz = 0;
           if (k <= 3 && pauli_form(cm.data(), d, false, px, pz)) so.aux = uint8_t(kAuxPauli | px | (pz << 3));
           ps.coef.insert(ps.coef.end(), cm.begin(), cm.end());
@@ -382,7 +406,7 @@ uint32_t op_budget(const PlanOptions &opt) {
 // that copy).
 struct OpInfo {
   uint64_t T, A, tm;  // non-diagonal, touched and target bits
-  uint32_t coef;
+  uint32_t coef, slot;
   bool diag, fits, inner;
 };
 
@@ -399,6 +423,7 @@ struct OpTable {
     f.diag = SweepBuilder::is_diag(op);
     f.fits = fusable_size(op, opt);
     f.inner = op.kind == kOpInner;
+    f.slot = op.slot;
   }
 };
 
@@ -406,7 +431,8 @@ struct OpTable {
 // the collection below, without growing S).
 uint32_t absorbed(const std::vector<const HostOp *> &rem, size_t head, uint64_t S, uint32_t n,
                   const PlanOptions &opt, size_t window, const OpTable &tab) {
-  uint32_t cnt = 0, ncoef = 0, ninner = 0;
+  uint32_t cnt = 0, ncoef = 0;
+  InnerSlotSet inner;
   const uint32_t max_ops = op_budget(opt);
   uint64_t blockT = 0, blockA = 0;
   size_t skipped = 0;
@@ -417,11 +443,11 @@ uint32_t absorbed(const std::vector<const HostOp *> &rem, size_t head, uint64_t 
     const bool diag = f.diag;
     const uint32_t c = f.coef;
     const bool fits = f.fits && (diag || (f.tm & ~S) == 0) && cnt < max_ops &&
-                      ncoef + c <= uint32_t(kMaxCoef) && !(f.inner && ninner >= uint32_t(kMaxInner));
+                      ncoef + c <= uint32_t(kMaxCoef) && !(f.inner && !inner.fits(f.slot));
     if (commutes && fits) {
       ++cnt;
       ncoef += c;
-      if (f.inner) ++ninner;
+      if (f.inner) inner.add(f.slot);
       if (cnt >= max_ops) break;
       continue;
     }
@@ -718,7 +744,8 @@ std::vector<PlannedLaunch> plan_sweeps(const std::vector<HostOp> &ops, uint32_t 
       std::vector<const HostOp *> chosen;
       std::vector<size_t> chosen_idx, skipped_idx;
       uint64_t blockT = 0, blockAll = 0;
-      uint32_t ncoef = 0, ninner = 0;
+      uint32_t ncoef = 0;
+      InnerSlotSet inner;
       size_t i = head;
       for (; i < rem.size(); ++i) {
         const HostOp &op = *rem[i];
@@ -729,13 +756,13 @@ std::vector<PlannedLaunch> plan_sweeps(const std::vector<HostOp> &ops, uint32_t 
         const uint32_t c = f.coef;
         const bool fits = f.fits && (diag || uint32_t(popc64(S | f.tm)) <= m) &&
                           chosen.size() < size_t(sb.max_ops) && ncoef + c <= uint32_t(kMaxCoef) &&
-                          !(f.inner && ninner >= uint32_t(kMaxInner));
+                          !(f.inner && !inner.fits(f.slot));
         if (commutes && fits) {
           if (!diag) S |= f.tm;
           chosen.push_back(&op);
           chosen_idx.push_back(i);
           ncoef += c;
-          if (f.inner) ++ninner;
+          if (f.inner) inner.add(f.slot);
           if (chosen.size() >= size_t(sb.max_ops)) {
             ++i;
             break;
@@ -784,7 +811,7 @@ std::vector<PlannedLaunch> plan_sweeps(const std::vector<HostOp> &ops, uint32_t 
       sb.ops = order;
       for (const HostOp *op : order) {
         sb.ncoef += SweepBuilder::coef_count(*op);
-        if (op->kind == kOpInner) ++sb.ninner;
+        if (op->kind == kOpInner) sb.inner.add(op->slot);
       }
       PlannedLaunch pl;
       pl.is_sweep = true;
@@ -914,7 +941,7 @@ bool rebuild_sweep(const SweepRecipe &r, const std::vector<HostOp> &ops, uint32_
     if (i >= ops.size()) return false;
     sb.ops.push_back(&ops[i]);
     sb.ncoef += SweepBuilder::coef_count(ops[i]);
-    if (ops[i].kind == kOpInner) ++sb.ninner;
+    if (ops[i].kind == kOpInner) sb.inner.add(ops[i].slot);
   }
   out = sb.finish();
   out.recipe = r;
