@@ -321,7 +321,7 @@ def kernel_tour():
     st.apply_ops(circuits.random_mix(n, 8, seed=SEED))  # gate_kernel, one launch per gate
     st.flush()
     terms = circuits.random_pauli_hamiltonian(n, 16, seed=SEED)
-    e = st.expectation(terms)  # pauli_expect_kernel
+    e = st.expectation(terms)  # pauli_expect_tiles
     st.close()
     ops, qterms, theta = qaoa_workload(22, 2)
     ws = adjoint.Workspace(22)

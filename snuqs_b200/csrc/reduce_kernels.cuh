@@ -12,8 +12,9 @@
 // Terms are grouped by (x, ny mod 2).  For x != 0 the pair (i, i^x), i with
 // the top bit of x clear, contributes (-1)^popc(i&zy) * q(i) with
 // q = 2 Re(conj(psi_i) psi_j) (ny even) or 2 Im(...) (ny odd); the host folds
-// the weight and the (-i)^ny phase into one real factor per term, so a group
-// costs one read of the state and the kernel needs one FP64 accumulator.
+// the weight and the (-i)^ny phase into one real factor per term.  The kernels
+// over whole states are in pauli_tiles.cuh; PauliParams serves the ones that
+// read a state of one tile or apply the sum to it.
 #pragma once
 #ifndef __CUDACC_RTC__
 #include <cuda_runtime.h>
@@ -58,48 +59,6 @@ __device__ __forceinline__ double block_sum(double v) {
   }
   __syncthreads();
   return v;  // valid in thread 0
-}
-
-// partial[blockIdx.x] (+)= this block's share of sum_groups sum_pairs q * W.
-template <typename Real>
-__global__ void __launch_bounds__(kReduceThreads)
-    pauli_expect_kernel(const typename Vec2<Real>::T *__restrict__ psi,
-                        const __grid_constant__ PauliParams P, double *__restrict__ partial,
-                        int accumulate) {
-  using C2 = typename Vec2<Real>::T;
-  double acc = 0.0;
-  const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
-  for (uint32_t gi = 0; gi < P.ngroups; ++gi) {
-    const PauliGroup &G = P.g[gi];
-    if (G.x == 0) {
-      const uint64_t N = uint64_t(1) << P.n;
-      for (uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < N; i += stride) {
-        const C2 a = psi[i];
-        const double q = double(a.x) * double(a.x) + double(a.y) * double(a.y);
-        double w = 0.0;
-        for (uint32_t t = G.t0; t < G.t1; ++t)
-          w += (__popcll(i & P.zy[t]) & 1) ? -P.f[t] : P.f[t];
-        acc = fma(q, w, acc);
-      }
-    } else {
-      const uint32_t hb = 63 - __clzll(G.x);
-      const uint64_t N = uint64_t(1) << (P.n - 1);
-      for (uint64_t h = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; h < N; h += stride) {
-        const uint64_t i = insert_zero(h, hb), j = i ^ G.x;
-        const C2 a = psi[i], b = psi[j];
-        // conj(a) * b
-        const double zr = double(a.x) * double(b.x) + double(a.y) * double(b.y);
-        const double zi = double(a.x) * double(b.y) - double(a.y) * double(b.x);
-        const double q = 2.0 * (G.odd ? zi : zr);
-        double w = 0.0;
-        for (uint32_t t = G.t0; t < G.t1; ++t)
-          w += (__popcll(i & P.zy[t]) & 1) ? -P.f[t] : P.f[t];
-        acc = fma(q, w, acc);
-      }
-    }
-  }
-  const double s = block_sum(acc);
-  if (threadIdx.x == 0) partial[blockIdx.x] = accumulate ? partial[blockIdx.x] + s : s;
 }
 
 // out[0] = sum of partial[0..n) in a fixed order (deterministic).
