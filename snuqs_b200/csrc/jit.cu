@@ -324,11 +324,14 @@ std::vector<int> thread_positions(const SweepPhase &ph, int m, bool c64, bool di
 // Ops whose coefficients are read from a shared-memory copy rather than the
 // parameter block: a diagonal op whose coefficient index depends on tile bits
 // that differ across the lanes (a lane-divergent constant read serialises),
-// and dense matrices, whose many coefficients are re-read for every register
-// group (one 16-byte shared load per complex entry beats two constant loads;
-// measured 5x cheaper per 2-qubit dense gate on B200).
-bool lane_indexed(const SweepOp &op) {
-  if (op.kind == kSwDense) return true;
+// and dense matrices of complex128 or of more than two qubits.  Those of
+// complex64 and at most two qubits are constant-bank operands of the FMAs:
+// no shared read and no coefficient registers, and fewer register operands
+// per FMA (the sweeps of a 27-qubit volume circuit 33.5 ms; with shared
+// reads 37.6 ms, 70 % of the issue slots used at 62 % of the FMA rate).  An
+// FP64 FMA gains nothing from it (26 qubits complex128: 34.3 against 33.1 ms).
+bool lane_indexed(const SweepOp &op, bool c64) {
+  if (op.kind == kSwDense) return !c64 || __builtin_popcount(op.vmask) > 2;
   if (op.kind != kSwDiag) return false;
   for (int t = 0; t < op.ndt; ++t)
     if (op.dsrc[t] != kSrcGlobal) return true;
@@ -766,7 +769,7 @@ JitShape jit_shape(const PlannedSweep &ps, bool c64, bool multi = false) {
   }();
   const bool dload_on = dload_env < 0 ? (!c64 || jit_early()) : dload_env == 1;
   JitShape j;
-  for (const SweepOp &op : ps.op) j.smem_coef |= lane_indexed(op);
+  for (const SweepOp &op : ps.op) j.smem_coef |= lane_indexed(op, c64);
   j.dload = dload_on && (ps.h.flags & kDirectLoad);
   j.dstore = (ps.h.flags & kDirectStore) != 0;
   // A one-phase remapping sweep cannot place its lanes for both a coalesced
@@ -879,7 +882,7 @@ std::string jit_body(const PlannedSweep &ps, bool c64, int minb, bool multi, boo
       s << "      Ph::gather(A, tile, jb);\n";
     one_state_ops_src(ps.op.data(), ph, R, c64, [&](const SweepOp &o) {
       std::ostringstream c;
-      if (multi || lane_indexed(o))
+      if (multi || lane_indexed(o, c64))
         c << "(coef + " << o.coef << ")";
       else
         c << "ParamCoef<" << R << ", " << o.coef << ">{P.coef}";
