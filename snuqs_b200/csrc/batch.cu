@@ -23,6 +23,7 @@
 #include "../../include/snuqs_b200.h"
 #include "adjoint_plan.h"
 #include "batch_energy.cuh"
+#include "batch_gradient.cuh"
 #include "batch_kernels.cuh"
 #include "host_ops.h"
 #include "jit.h"
@@ -126,6 +127,7 @@ struct sq_batch {
   std::vector<sq::PauliTilePlan> ham_tiles;  // the same sums, for the energy pass of streamed states
   std::vector<uint32_t> ham_n;
   std::vector<Circ> circs;
+  DevBuf d_rows, d_entries;  // gradient runs as multi-state sweeps: inner-product rows, their index
   DevBuf d_pool, d_plans, d_table, d_hams, d_tiles, d_energy, d_counter, d_occ, d_def, d_part;
   HostBuf h_plans, h_table, h_energy, h_occ, h_def;
   std::vector<uint32_t> deferred;  // table positions whose energy the grid-wide pass computes
@@ -408,6 +410,10 @@ std::vector<sq::PlannedSweep> unpack_sweeps(const std::vector<unsigned char> &p,
     ps.ph.assign(ph, ph + rec.h.nphases);
     ps.op.assign(op, op + rec.nops);
     ps.coef.assign(rec.h.ncoef, cplx(0.0, 0.0));
+    if (rec.inner_off) {
+      const auto *g = reinterpret_cast<const uint32_t *>(p.data() + off + rec.inner_off);
+      ps.inner_global.assign(g + 1, g + 1 + g[0]);
+    }
     out.push_back(std::move(ps));
     coef_at.push_back(off + rec.coef_off);
     off += rec.bytes;
@@ -923,7 +929,7 @@ int run_impl(sq_batch *b, double *energies, cudaStream_t st) {
 template <typename Real>
 bool plan_gradient_circuit(const Circ &c, uint32_t m, std::vector<unsigned char> &out, uint32_t &nfwd,
                            uint32_t &nrev, std::vector<std::pair<int32_t, double>> &occ, std::string &err,
-                           PlanShare *share = nullptr) {
+                           PlanShare *share = nullptr, bool multi = false) {
   try {
     sq::AdjointPlan ap;
     sq::build_adjoint(c.ops.data(), uint32_t(c.ops.size()), c.n, ap);
@@ -934,6 +940,13 @@ bool plan_gradient_circuit(const Circ &c, uint32_t m, std::vector<unsigned char>
     ropt.tile_bits = m;
     ropt.reg_bits = sq::kAdjRegBits;
     ropt.max_dense_k = sq::kAdjRegBits;
+    if (multi) {
+      // Multi-state sweeps: the tiles of the single-state passes.
+      ropt.tile_bits = uint32_t(sizeof(Real) == 4 ? sq::kAdjTileBitsC64[2] : sq::kAdjTileBitsC128[2]);
+      fopt.tile_bits = batch_default_bits<Real>();
+      fopt.low_bits = sq::auto_low_bits(sizeof(Real) == 4, c.n, fopt.tile_bits);
+      fopt.select = ropt.select = multi_select();
+    }
     const auto fplan = share ? share->plan(ap.forward, c.n, fopt) : sq::plan_sweeps(ap.forward, c.n, fopt);
     const auto rplan = share ? share->plan(ap.reverse, c.n, ropt) : sq::plan_sweeps(ap.reverse, c.n, ropt);
     nfwd = nrev = 0;
@@ -982,6 +995,66 @@ bool uniform_plans(const sq_batch *b, const std::vector<std::vector<unsigned cha
   return true;
 }
 
+// Launch description of a gradient run as multi-state sweeps.
+struct MultiGradient {
+  std::vector<MultiSweep> fwd, rev;
+  std::vector<std::vector<uint32_t>> inner;  // per reverse sweep: occurrence of each slot
+  std::vector<uint32_t> tile_bits;           // per reverse sweep
+  bool zero_first = false;
+};
+
+// Kernels of the sweeps of one circuit's packed gradient plan in their
+// multi-state forms; false when one cannot be had.
+template <typename Real>
+bool multi_gradient_kernels(const std::vector<unsigned char> &plan, uint32_t nfwd, MultiGradient &G) {
+  constexpr bool c64 = sizeof(Real) == 4;
+  std::vector<uint64_t> coef_at;
+  const std::vector<sq::PlannedSweep> sweeps = unpack_sweeps(plan, coef_at);
+  const uint32_t MF = batch_default_bits<Real>();
+  std::vector<const sq::PlannedSweep *> fwd, zero, rev;
+  for (size_t k = 0; k < sweeps.size(); ++k) {
+    const sq::PlannedSweep &ps = sweeps[k];
+    if (k >= nfwd) rev.push_back(&ps);
+    else if (ps.h.m != MF) return false;
+    else if (k == 0 && !sq::jit_body(ps, c64, sq::jit_minb(c64, MF), true, true).empty()) zero.push_back(&ps);
+    else fwd.push_back(&ps);
+  }
+  sq::jit_prepare_multi(fwd, c64, zero);
+  sq::jit_prepare_madjoint(rev, c64);
+  for (size_t k = 0; k < sweeps.size(); ++k) {
+    const sq::PlannedSweep &ps = sweeps[k];
+    const bool r = k >= nfwd;
+    MultiSweep w;
+    std::string err;
+    if (r) {
+      w.fn = sq::jit_madjoint_kernel(ps, c64, err);
+      w.smem = sq::jit_adjoint_smem(ps, c64);
+    } else {
+      const bool z = k == 0 && !zero.empty();
+      if (z) w.fn = sq::jit_msweep_kernel(ps, c64, err, true);
+      if (z && w.fn) G.zero_first = true;
+      if (!w.fn) w.fn = sq::jit_msweep_kernel(ps, c64, err);
+      w.smem = sq::jit_msweep_smem(ps, c64);
+    }
+    w.ncoef = ps.h.ncoef;
+    w.coef_at = coef_at[k];
+    const int threads = 1 << (ps.h.m - uint32_t(r ? sq::kAdjRegBits : sq::kRegBits));
+    if (!w.fn ||
+        cudaFuncSetAttribute(w.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(w.smem)) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&w.per_sm, w.fn, threads, w.smem) != cudaSuccess) {
+      cudaGetLastError();
+      return false;
+    }
+    w.per_sm = std::max(w.per_sm, 1);
+    (r ? G.rev : G.fwd).push_back(w);
+    if (r) {
+      G.inner.push_back(ps.inner_global);
+      G.tile_bits.push_back(ps.h.m);
+    }
+  }
+  return true;
+}
+
 template <typename Real>
 int run_gradient_impl(sq_batch *b, uint32_t n_params, double *energies, double *grads, cudaStream_t st) {
   using C2 = typename sq::Vec2<Real>::T;
@@ -995,6 +1068,7 @@ int run_gradient_impl(sq_batch *b, uint32_t n_params, double *energies, double *
   b->planned_version = ~uint64_t(0);
   if (b->graph) cudaGraphExecDestroy(b->graph);
   b->graph = nullptr;
+  MultiGradient multi;
   std::vector<std::vector<unsigned char>> packed(nc);
   std::vector<uint32_t> nfwd(nc, 0), nrev(nc, 0);
   std::vector<std::vector<std::pair<int32_t, double>>> occs(nc);
@@ -1002,14 +1076,37 @@ int run_gradient_impl(sq_batch *b, uint32_t n_params, double *energies, double *
   std::vector<char> ok(nc, 0);
   std::atomic<size_t> next{0};
   const unsigned nth = std::max(1u, std::min(16u, std::thread::hardware_concurrency()));
-  PlanShare share;
-  std::vector<std::thread> workers;
-  for (unsigned t = 0; t < nth; ++t)
-    workers.emplace_back([&]() {
-      for (size_t i = next++; i < nc; i = next++)
-        ok[i] = plan_gradient_circuit<Real>(b->circs[i], M, packed[i], nfwd[i], nrev[i], occs[i], errs[i], &share);
-    });
-  for (auto &th : workers) th.join();
+  // Circuits of one size above the tile are planned for multi-state sweeps
+  // (parameter sets of one circuit); when their plans turn out to differ, for
+  // the kernel that runs one circuit per CTA.
+  bool try_multi = multi_enabled() && b->circs[0].n > M && b->circs[0].n >= sq::kApplyBits;
+  for (size_t i = 1; i < nc; ++i) try_multi = try_multi && b->circs[i].n == b->circs[0].n;
+  auto plan_all = [&](bool as_multi) {
+    PlanShare share;
+    next = 0;
+    std::vector<std::thread> workers;
+    for (unsigned t = 0; t < nth; ++t)
+      workers.emplace_back([&]() {
+        for (size_t i = next++; i < nc; i = next++) {
+          packed[i].clear();
+          occs[i].clear();
+          ok[i] = plan_gradient_circuit<Real>(b->circs[i], M, packed[i], nfwd[i], nrev[i], occs[i], errs[i], &share,
+                                              as_multi);
+        }
+      });
+    for (auto &th : workers) th.join();
+  };
+  plan_all(try_multi);
+  if (try_multi) {
+    bool fine = true;
+    for (size_t i = 0; i < nc; ++i) fine = fine && ok[i];
+    fine = fine && uniform_plans<Real>(b, packed, nfwd, nrev, occs, M) &&
+           multi_gradient_kernels<Real>(packed[0], nfwd[0], multi);
+    if (!fine) {
+      try_multi = false;
+      plan_all(false);
+    }
+  }
   for (size_t i = 0; i < nc; ++i) {
     if (!ok[i]) return fail(SQ_ERR_UNSUPPORTED, errs[i]);
     for (const auto &o : occs[i])
@@ -1020,7 +1117,7 @@ int run_gradient_impl(sq_batch *b, uint32_t n_params, double *energies, double *
   // Circuits that all share one plan structure (many parameter sets of one
   // circuit) and stream their states get a JIT-specialised kernel.
   const void *jit_fn = nullptr;
-  if (uniform_plans<Real>(b, packed, nfwd, nrev, occs, M)) {
+  if (!try_multi && uniform_plans<Real>(b, packed, nfwd, nrev, occs, M)) {
     // Looked up by plan structure: a repeated gradient run of the same
     // circuit skips generating (and hashing) the kernel's source.
     static std::mutex memo_mu;
@@ -1056,7 +1153,10 @@ int run_gradient_impl(sq_batch *b, uint32_t n_params, double *energies, double *
   std::vector<uint64_t> psi_off(nc, 0), lam_off(nc, 0), occ_off(nc, 0);
   for (uint32_t id : b->order) {
     const Circ &c = b->circs[id];
-    if (c.n > M) {
+    if (try_multi) {  // K psi, then K lambda
+      psi_off[id] = pool_amps;
+      pool_amps += uint64_t(1) << c.n;
+    } else if (c.n > M) {
       psi_off[id] = pool_amps;
       lam_off[id] = pool_amps + (uint64_t(1) << c.n);
       pool_amps += uint64_t(2) << c.n;
@@ -1064,6 +1164,8 @@ int run_gradient_impl(sq_batch *b, uint32_t n_params, double *energies, double *
     occ_off[id] = nocc;
     nocc += occs[id].size();
   }
+  const uint64_t lam0 = pool_amps;
+  if (try_multi) pool_amps *= 2;
   size_t plan_bytes = 0;
   for (size_t i = 0; i < nc; ++i) plan_bytes += packed[i].size();
   SQB_CUDA(cudaSetDevice(b->device));
@@ -1102,45 +1204,130 @@ int run_gradient_impl(sq_batch *b, uint32_t n_params, double *energies, double *
     t.plan_off = off;
     off += packed[id].size();
   }
-  const void *fn = jit_fn ? jit_fn : batch_adj_fn<Real>(M);
-  const uint32_t L = uint32_t(sq::sweep_low_bits(int(M)));
-  const int threads = 1 << (M - sq::kAdjRegBits);
-  const size_t nw = size_t(threads + 31) / 32;
-  const size_t smem = 4 * (size_t(1) << M) * sizeof(C2) + size_t(sq::kMaxCoef) * sizeof(C2) +
-                      (jit_fn ? 0 : (size_t(1) << (M - L)) * sizeof(uint64_t)) +
-                      nw * sq::kMaxInner * sizeof(double2);
-  b->last_jit = jit_fn != nullptr;
-  if (jit_fn) sq::jit_note_launch(true);
-  SQB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-  int per_sm = 0, sms = 0;
-  SQB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, smem));
+  int sms = 0;
   SQB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->device));
-  const uint32_t grid = uint32_t(std::max<uint64_t>(
-      1, std::min<uint64_t>(nc, uint64_t(std::max(per_sm, 1)) * uint64_t(sms))));
   if (!b->ev0) {
     SQB_CUDA(cudaEventCreate(&b->ev0));
     SQB_CUDA(cudaEventCreate(&b->ev1));
   }
-  sq::BatchParams P;
-  std::memset(&P, 0, sizeof(P));
-  P.circuits = static_cast<const sq::BatchCircuit *>(b->d_table.p);
-  P.plans = static_cast<const unsigned char *>(b->d_plans.p);
-  P.hams = static_cast<const sq::PauliParams *>(b->d_hams.p);
-  P.ncircuits = uint32_t(nc);
-  P.counter = static_cast<unsigned *>(b->d_counter.p);
-  P.energies = static_cast<double *>(b->d_energy.p);
   C2 *poolp = static_cast<C2 *>(b->d_pool.p);
   double2 *occp = static_cast<double2 *>(b->d_occ.p);
-  void *args[] = {&poolp, &P, &occp};
+  uint32_t grid = 0;
   SQB_CUDA(cudaMemcpyAsync(b->d_plans.p, b->h_plans.p, plan_bytes, cudaMemcpyHostToDevice, st));
   SQB_CUDA(cudaMemcpyAsync(b->d_table.p, b->h_table.p, nc * sizeof(sq::BatchCircuit),
                            cudaMemcpyHostToDevice, st));
-  SQB_CUDA(cudaMemsetAsync(b->d_counter.p, 0, sizeof(unsigned), st));
-  SQB_CUDA(cudaMemsetAsync(b->d_occ.p, 0, std::max<uint64_t>(nocc, 1) * sizeof(double2), st));
-  SQB_CUDA(cudaEventRecord(b->ev0, st));
-  SQB_CUDA(cudaLaunchKernel(fn, dim3(grid), dim3(threads), args, smem, st));
-  SQB_CUDA(cudaGetLastError());
-  SQB_CUDA(cudaEventRecord(b->ev1, st));
+  if (try_multi) {
+    const uint32_t n = b->circs[0].n;
+    const uint64_t total = uint64_t(nc) << n;
+    C2 *lamp = poolp + lam0;
+    auto params = [&](const MultiSweep &w, uint32_t m) {
+      sq::MultiParams Q;
+      Q.coefs = static_cast<const unsigned char *>(b->d_plans.p) + w.coef_at;
+      Q.stride = packed[0].size();
+      Q.tile_shift = n - m;
+      Q.tiles = uint64_t(nc) << Q.tile_shift;
+      Q.ncoef = w.ncoef;
+      return Q;
+    };
+    // Rows of every reverse sweep, and the entries of each occurrence.
+    const uint32_t nocc1 = uint32_t(occs[0].size());
+    std::vector<std::vector<sq::GradientEntry>> by_occ(nocc1);
+    std::vector<uint64_t> row_at(multi.rev.size());
+    std::vector<uint32_t> rows_per(multi.rev.size()), grids(multi.rev.size());
+    uint64_t nrows = 0;
+    for (size_t k = 0; k < multi.rev.size(); ++k) {
+      const sq::MultiParams Q = params(multi.rev[k], multi.tile_bits[k]);
+      grids[k] = uint32_t(std::min<uint64_t>(Q.tiles, uint64_t(multi.rev[k].per_sm) * uint64_t(sms)));
+      const uint64_t per = (Q.tiles + grids[k] - 1) / grids[k];
+      rows_per[k] = uint32_t(((uint64_t(1) << Q.tile_shift) + per - 1) / per + 1);
+      row_at[k] = nrows;
+      nrows += uint64_t(nc) * rows_per[k] * sq::kMaxInner;
+      for (size_t s = 0; s < multi.inner[k].size(); ++s)
+        by_occ[multi.inner[k][s]].push_back({row_at[k], per, rows_per[k], Q.tile_shift, uint32_t(s), 0});
+    }
+    std::vector<sq::GradientEntry> entries;
+    std::vector<uint32_t> first{0};
+    for (const auto &v : by_occ) {
+      entries.insert(entries.end(), v.begin(), v.end());
+      first.push_back(uint32_t(entries.size()));
+    }
+    const size_t ebytes = entries.size() * sizeof(sq::GradientEntry), fbytes = first.size() * sizeof(uint32_t);
+    const uint32_t apply_blocks = uint32_t(total >> sq::kApplyBits);
+    if (int s = b->d_rows.ensure(std::max<uint64_t>(nrows, 1) * sizeof(double))) return s;
+    if (int s = b->d_entries.ensure(ebytes + fbytes + 16)) return s;
+    if (int s = b->d_part.ensure(apply_blocks * sizeof(double))) return s;
+    // Pageable sources: staged before the calls return.
+    if (ebytes) SQB_CUDA(cudaMemcpyAsync(b->d_entries.p, entries.data(), ebytes, cudaMemcpyHostToDevice, st));
+    SQB_CUDA(cudaMemcpyAsync(static_cast<char *>(b->d_entries.p) + ebytes, first.data(), fbytes,
+                             cudaMemcpyHostToDevice, st));
+    b->last_jit = true;
+    sq::jit_note_launch(true);
+    SQB_CUDA(cudaEventRecord(b->ev0, st));
+    if (!multi.zero_first)
+      sq::batch_group_init<Real><<<uint32_t(std::min<uint64_t>((total + 255) / 256, uint64_t(sms) * 8)), 256, 0, st>>>(
+          poolp, total, n);
+    const uint32_t MF = batch_default_bits<Real>();
+    for (const MultiSweep &w : multi.fwd) {
+      sq::MultiParams Q = params(w, MF);
+      void *margs[] = {&poolp, &Q};
+      const uint64_t mg = std::min<uint64_t>(Q.tiles, uint64_t(w.per_sm) * uint64_t(sms));
+      SQB_CUDA(cudaLaunchKernel(w.fn, dim3(unsigned(mg)), dim3(1u << (MF - sq::kRegBits)), margs, w.smem, st));
+      grid = std::max(grid, uint32_t(mg));
+    }
+    double *partp = static_cast<double *>(b->d_part.p);
+    sq::batch_apply_kernel<Real><<<apply_blocks, sq::kReduceThreads, 0, st>>>(
+        poolp, lamp, static_cast<const sq::BatchCircuit *>(b->d_table.p),
+        static_cast<const sq::PauliParams *>(b->d_hams.p), n, partp);
+    sq::batch_apply_finalize<<<unsigned(nc), sq::kReduceThreads, 0, st>>>(partp, 1u << (n - sq::kApplyBits),
+                                                                         static_cast<double *>(b->d_energy.p));
+    for (size_t k = 0; k < multi.rev.size(); ++k) {
+      const MultiSweep &w = multi.rev[k];
+      const uint32_t m = multi.tile_bits[k];
+      sq::MultiParams Q = params(w, m);
+      double *rows = static_cast<double *>(b->d_rows.p) + row_at[k];
+      uint32_t nslots = uint32_t(multi.inner[k].size());
+      void *margs[] = {&poolp, &lamp, &Q, &rows, &rows_per[k], &nslots};
+      SQB_CUDA(cudaLaunchKernel(w.fn, dim3(grids[k]), dim3(1u << (m - sq::kAdjRegBits)), margs, w.smem, st));
+    }
+    if (nocc1) {
+      const auto *ent = static_cast<const sq::GradientEntry *>(b->d_entries.p);
+      const auto *fst = reinterpret_cast<const uint32_t *>(static_cast<const char *>(b->d_entries.p) + ebytes);
+      sq::gradient_reduce_kernel<<<unsigned(nc) * nocc1, 128, 0, st>>>(static_cast<const double *>(b->d_rows.p), ent,
+                                                                      fst, nocc1, occp);
+    }
+    SQB_CUDA(cudaGetLastError());
+    SQB_CUDA(cudaEventRecord(b->ev1, st));
+  } else {
+    const void *fn = jit_fn ? jit_fn : batch_adj_fn<Real>(M);
+    const uint32_t L = uint32_t(sq::sweep_low_bits(int(M)));
+    const int threads = 1 << (M - sq::kAdjRegBits);
+    const size_t nw = size_t(threads + 31) / 32;
+    const size_t smem = 4 * (size_t(1) << M) * sizeof(C2) + size_t(sq::kMaxCoef) * sizeof(C2) +
+                        (jit_fn ? 0 : (size_t(1) << (M - L)) * sizeof(uint64_t)) +
+                        nw * sq::kMaxInner * sizeof(double2);
+    b->last_jit = jit_fn != nullptr;
+    if (jit_fn) sq::jit_note_launch(true);
+    SQB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    int per_sm = 0;
+    SQB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, smem));
+    grid = uint32_t(std::max<uint64_t>(
+        1, std::min<uint64_t>(nc, uint64_t(std::max(per_sm, 1)) * uint64_t(sms))));
+    sq::BatchParams P;
+    std::memset(&P, 0, sizeof(P));
+    P.circuits = static_cast<const sq::BatchCircuit *>(b->d_table.p);
+    P.plans = static_cast<const unsigned char *>(b->d_plans.p);
+    P.hams = static_cast<const sq::PauliParams *>(b->d_hams.p);
+    P.ncircuits = uint32_t(nc);
+    P.counter = static_cast<unsigned *>(b->d_counter.p);
+    P.energies = static_cast<double *>(b->d_energy.p);
+    void *args[] = {&poolp, &P, &occp};
+    SQB_CUDA(cudaMemsetAsync(b->d_counter.p, 0, sizeof(unsigned), st));
+    SQB_CUDA(cudaMemsetAsync(b->d_occ.p, 0, std::max<uint64_t>(nocc, 1) * sizeof(double2), st));
+    SQB_CUDA(cudaEventRecord(b->ev0, st));
+    SQB_CUDA(cudaLaunchKernel(fn, dim3(grid), dim3(threads), args, smem, st));
+    SQB_CUDA(cudaGetLastError());
+    SQB_CUDA(cudaEventRecord(b->ev1, st));
+  }
   SQB_CUDA(cudaMemcpyAsync(b->h_energy.p, b->d_energy.p, nc * sizeof(double), cudaMemcpyDeviceToHost, st));
   SQB_CUDA(cudaMemcpyAsync(b->h_occ.p, b->d_occ.p, std::max<uint64_t>(nocc, 1) * sizeof(double2),
                            cudaMemcpyDeviceToHost, st));
@@ -1188,6 +1375,8 @@ int sq_batch_destroy(sq_batch *b) {
   b->d_plans.release();
   b->d_table.release();
   b->d_hams.release();
+  b->d_rows.release();
+  b->d_entries.release();
   b->d_tiles.release();
   b->d_energy.release();
   b->d_counter.release();

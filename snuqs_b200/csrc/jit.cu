@@ -366,7 +366,7 @@ std::string inner_slots(const SweepOp *ops, size_t nops, bool finish, int NT) {
   std::ostringstream s;
   for (uint32_t i = 0; i < std::min(n, kRegSlots); ++i)
     if (finish)
-      s << " jit_inner_acc<" << NT << ", " << i << ">(acc, ip" << i << ");";
+      s << " jit_inner_acc<" << NT << ", " << i << ">(acc, ip" << i << "); ip" << i << " = 0.0;";
     else
       s << " double ip" << i << " = 0.0;";
   return s.str();
@@ -909,23 +909,27 @@ std::string jit_source(const PlannedSweep &ps, bool c64, int minb, bool multi, b
 
 // Source of the JIT kernel of one reverse (two-state) adjoint sweep; empty
 // when the sweep holds an op the generated form does not cover (the generic
-// adjoint kernel then runs it).
-std::string jit_adjoint_body(const PlannedSweep &ps, bool c64, int minb) {
+// adjoint kernel then runs it).  multi: the form over K pairs of states
+// (sq_jit_madjoint).
+std::string jit_adjoint_body(const PlannedSweep &ps, bool c64, int minb, bool multi) {
   const char *R = c64 ? "float" : "double";
   const int M = int(ps.h.m);
   const int NT = 1 << (M - kAdjRegBits);
   std::ostringstream s;
-  s << "extern \"C\" __global__ void __launch_bounds__(" << NT << ", " << minb
-    << ")\nsq_jit_adjoint(Vec2<" << R << ">::T *__restrict__ psi, Vec2<" << R
-    << ">::T *__restrict__ lam, const __grid_constant__ SweepParams<" << R
-    << "> P, double2 *__restrict__ partials) {\n";
+  s << "extern \"C\" __global__ void __launch_bounds__(" << NT << ", " << minb << ")\nsq_jit_"
+    << (multi ? "madjoint" : "adjoint") << "(Vec2<" << R << ">::T *__restrict__ psi, Vec2<" << R
+    << ">::T *__restrict__ lam, ";
+  if (multi)
+    s << "const __grid_constant__ MultiParams Q, double *__restrict__ rows, uint32_t rows_per, uint32_t nslots) {\n";
+  else
+    s << "const __grid_constant__ SweepParams<" << R << "> P, double2 *__restrict__ partials) {\n";
   s << "  using C2 = Vec2<" << R << ">::T;\n";
   s << "  using Tile = JitTile<" << M << ", " << ps.h.l;
   for (uint32_t i = 0; i < ps.h.m - ps.h.l; ++i) s << ", " << int(ps.h.hi[i]);
   s << ">;\n";
   s << " " << inner_slots(ps.op.data(), ps.op.size(), false, NT) << "\n";
-  s << "  jit_adjoint_sweep<" << R << ", " << M
-    << ", Tile>(psi, lam, P, partials, [&](C2 *ft, C2 *lt, const C2 *coef, uint64_t gbase, double2 *acc) {\n";
+  s << "  jit_" << (multi ? "m" : "") << "adjoint_sweep<" << R << ", " << M << ", Tile>(psi, lam, "
+    << (multi ? "Q, rows, rows_per, nslots" : "P, partials") << ", [&](C2 *ft, C2 *lt, const C2 *coef, uint64_t gbase, double2 *acc) {\n";
   for (uint32_t p = 0; p < ps.h.nphases; ++p) {
     const SweepPhase &ph = ps.ph[p];
     s << "    {\n      using Ph = JitPhase2<" << R << ", " << M << ", Tile, " << int(ph.reg[0]) << ", "
@@ -1145,6 +1149,17 @@ Entry *adjoint_entry(const PlannedSweep &ps, bool c64) {
   return e;
 }
 
+Entry *madjoint_entry(const PlannedSweep &ps, bool c64) {
+  const PlanKey k = plan_key(ps, c64, 4);
+  bool found = false;
+  Entry *e = plan_lookup(k, &found);
+  if (found) return e;
+  const std::string body = jit_adjoint_body(ps, c64, jit_adjoint_minb(c64), true);
+  e = body.empty() ? nullptr : &get_entry(body, "sq_jit_madjoint");
+  plan_store(k, e);
+  return e;
+}
+
 Entry &sweep_entry(const PlannedSweep &ps, bool c64) {
   const PlanKey k = plan_key(ps, c64, 0);
   bool found = false;
@@ -1179,6 +1194,15 @@ const void *jit_adjoint_kernel(const PlannedSweep &ps, bool c64, std::string &er
   return reinterpret_cast<const void *>(e->kernel);
 }
 
+const void *jit_madjoint_kernel(const PlannedSweep &ps, bool c64, std::string &err) {
+  Entry *e = madjoint_entry(ps, c64);
+  if (!e || e->failed) {
+    err = e ? e->err : "sweep not covered by the JIT adjoint form";
+    return nullptr;
+  }
+  return reinterpret_cast<const void *>(e->kernel);
+}
+
 // Compiles (in parallel) the kernels of structures not seen before.
 template <class F>
 void prepare_parallel(const std::vector<const PlannedSweep *> &sweeps, F make) {
@@ -1203,6 +1227,17 @@ void jit_prepare_adjoint(const std::vector<const PlannedSweep *> &sweeps, bool c
     if (!found) todo.push_back(ps);
   }
   prepare_parallel(todo, [&](const PlannedSweep &ps) { adjoint_entry(ps, c64); });
+}
+
+void jit_prepare_madjoint(const std::vector<const PlannedSweep *> &sweeps, bool c64) {
+  if (!jit_available() || sweeps.empty()) return;
+  std::vector<const PlannedSweep *> todo;
+  for (const auto *ps : sweeps) {
+    bool found = false;
+    plan_lookup(plan_key(*ps, c64, 4), &found);
+    if (!found) todo.push_back(ps);
+  }
+  prepare_parallel(todo, [&](const PlannedSweep &ps) { madjoint_entry(ps, c64); });
 }
 
 size_t jit_smem(const PlannedSweep &ps, bool c64) {

@@ -30,9 +30,13 @@ const void *jit_sweep_kernel(const PlannedSweep &ps, bool c64, std::string &err)
 // a parallel pre-compile of several sweeps.
 const void *jit_adjoint_kernel(const PlannedSweep &ps, bool c64, std::string &err);
 size_t jit_adjoint_smem(const PlannedSweep &ps, bool c64);
-std::string jit_adjoint_body(const PlannedSweep &ps, bool c64, int minb);
+std::string jit_adjoint_body(const PlannedSweep &ps, bool c64, int minb, bool multi = false);
 int jit_adjoint_minb(bool c64);
 void jit_prepare_adjoint(const std::vector<const PlannedSweep *> &sweeps, bool c64);
+// The same over K pairs of states that share the sweep's structure
+// (sq_jit_madjoint; shared memory as jit_adjoint_smem).
+const void *jit_madjoint_kernel(const PlannedSweep &ps, bool c64, std::string &err);
+void jit_prepare_madjoint(const std::vector<const PlannedSweep *> &sweeps, bool c64);
 // Batched gradients of circuits that share one packed plan structure
 // (`plan`: one circuit's packed records, nfwd forward then nrev reverse
 // sweeps, every sweep of m == M): the kernel (or nullptr with `err`), its

@@ -823,4 +823,97 @@ __device__ __forceinline__ void jit_adjoint_sweep(typename Vec2<Real>::T *__rest
     partials[size_t(blockIdx.x) * NW * kMaxInner + i] = acc[i];
 }
 
+// The two-state tile loop over the tiles of K pairs of states that share the
+// sweep's structure (MultiParams; psi and lambda each hold K states back to
+// back): one launch per reverse sweep for all parameter sets of one circuit,
+// instead of one CTA per circuit.  Each CTA takes a contiguous range of tiles;
+// when it crosses into the next state (and at its end) the inner products go
+// to a row of that state: rows[(c * rows_per + r) * kMaxInner + slot], with r
+// the CTA's number among those that touch state c.  finish(acc) adds the
+// per-thread sums to the warps' slots and clears them.
+template <typename Real, int M, class Tile, class Phases, class Finish>
+__device__ __forceinline__ void jit_madjoint_sweep(typename Vec2<Real>::T *__restrict__ psi,
+                                                   typename Vec2<Real>::T *__restrict__ lam, const MultiParams &Q,
+                                                   double *__restrict__ rows, uint32_t rows_per, uint32_t nslots,
+                                                   Phases phases, Finish finish) {
+  using C2 = typename Vec2<Real>::T;
+  constexpr int NT = 1 << (M - kAdjRegBits);
+  constexpr int NW = (NT + 31) / 32;
+  constexpr uint32_t TS = 1u << M;
+  constexpr uint32_t PER = TS / NT;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  C2 *fbufs = reinterpret_cast<C2 *>(smem_raw);
+  C2 *lbufs = fbufs + 2 * TS;
+  C2 *coef = lbufs + 2 * TS;
+  double2 *acc = reinterpret_cast<double2 *>(coef + ((Q.ncoef + 1) & ~1u));
+  const uint32_t tid = threadIdx.x;
+  auto clear = [&] {
+    for (uint32_t i = tid; i < NW * kMaxInner; i += NT) {
+      double2 z;
+      z.x = 0.0;
+      z.y = 0.0;
+      acc[i] = z;
+    }
+  };
+  const uint64_t per = (Q.tiles + gridDim.x - 1) / gridDim.x;
+  uint64_t t0, t1;
+  jit_multi_range(Q, t0, t1);
+  auto flush = [&](uint64_t c) {  // state c's sums of this CTA (uniform call)
+    finish(acc);
+    __syncthreads();
+    if (tid < nslots) {
+      double s = 0.0;
+      for (int w = 0; w < NW; ++w) s += acc[w * kMaxInner + tid].x;
+      const uint64_t r = blockIdx.x - (c << Q.tile_shift) / per;
+      rows[(c * rows_per + r) * kMaxInner + tid] = s;
+    }
+    __syncthreads();
+    clear();
+  };
+  clear();
+  const uint32_t s_tid = swz<Real>(tid);
+  const uint64_t toff = Tile::off(tid);
+  auto prefetch = [&](uint64_t t, C2 *fdst, C2 *ldst) {
+    const uint64_t g0 = Tile::base(t) | toff;
+#pragma unroll
+    for (uint32_t it = 0; it < PER; ++it) {
+      const uint64_t g = g0 | Tile::off(it * NT);
+      const uint32_t s = s_tid ^ swz<Real>(it * NT);
+      cp_async<sizeof(C2)>(fdst + s, psi + g);
+      cp_async<sizeof(C2)>(ldst + s, lam + g);
+    }
+  };
+  uint64_t cur_c = ~uint64_t(0);
+  uint32_t cur = 0;
+  if (t0 < t1) prefetch(t0, fbufs, lbufs);
+  cp_async_commit();
+  for (uint64_t t = t0; t < t1; ++t) {
+    C2 *ft = fbufs + cur * TS, *lt = lbufs + cur * TS;
+    if (t + 1 < t1) prefetch(t + 1, fbufs + (cur ^ 1) * TS, lbufs + (cur ^ 1) * TS);
+    cp_async_commit();
+    const uint64_t c = t >> Q.tile_shift;
+    if (c != cur_c) {  // uniform: the previous tile ended with a barrier
+      if (cur_c != ~uint64_t(0)) flush(cur_c);
+      jit_multi_coef<Real>(coef, Q, c);
+      cur_c = c;
+    }
+    cp_async_wait_prev();
+    __syncthreads();
+    const uint64_t gbase = Tile::base(t);
+    phases(ft, lt, coef, gbase, acc);
+    const uint64_t g0 = gbase | toff;
+#pragma unroll
+    for (uint32_t it = 0; it < PER; ++it) {
+      const uint64_t g = g0 | Tile::off(it * NT);
+      const uint32_t s = s_tid ^ swz<Real>(it * NT);
+      psi[g] = ft[s];
+      lam[g] = lt[s];
+    }
+    __syncthreads();
+    cur ^= 1;
+  }
+  asm volatile("cp.async.wait_all;\n" ::: "memory");
+  if (cur_c != ~uint64_t(0)) flush(cur_c);
+}
+
 }  // namespace sq
