@@ -633,7 +633,8 @@ void one_state_ops_src(const SweepOp *ops, const SweepPhase &ph, const char *R, 
     if (op.kind == kSwDiag)
       s << "{ " << diag_bits_src(op) << " " << tmpl << "(A, " << coef(op) << ", b); }\n";
     else
-      s << tmpl << "(A, " << coef(op) << ", " << int(op.rmask) << ", " << int(op.rval) << ");\n";
+      s << (op.kind == kSwDense && !lane_indexed(op, c64) ? "jit_" : "") << tmpl << "(A, " << coef(op) << ", "
+        << int(op.rmask) << ", " << int(op.rval) << ");\n";
   }
 }
 
