@@ -104,35 +104,6 @@ struct MultiSweep {
   uint64_t coef_at = 0;
 };
 
-// Plans shared between the circuits of one structure (many parameter sets of
-// one ansatz): the first circuit of a structure (op signature, qubits, plan
-// options) is planned, the others re-emit its plan with their own values
-// (sq::rebuild_plan), and fall back to planning when that fails.
-struct PlanShare {
-  using Key = std::tuple<uint64_t, uint64_t, uint64_t, uint32_t>;
-  std::mutex mu;
-  std::map<Key, std::shared_ptr<const std::vector<sq::PlannedLaunch>>> plans;
-
-  std::vector<sq::PlannedLaunch> plan(const std::vector<sq::HostOp> &ops, uint32_t n, const sq::PlanOptions &opt) {
-    const auto sig = sq::op_signature_hash(ops);
-    const Key key{sig.first, sig.second, sq::plan_options_key(opt), n};
-    std::shared_ptr<const std::vector<sq::PlannedLaunch>> have;
-    {
-      std::lock_guard<std::mutex> lk(mu);
-      auto it = plans.find(key);
-      if (it != plans.end()) have = it->second;
-    }
-    if (have) {
-      std::vector<sq::PlannedLaunch> p = *have;
-      if (sq::rebuild_plan(p, ops, n)) return p;
-    }
-    std::vector<sq::PlannedLaunch> p = sq::plan_sweeps(ops, n, opt);
-    std::lock_guard<std::mutex> lk(mu);
-    plans.emplace(key, std::make_shared<const std::vector<sq::PlannedLaunch>>(p));
-    return p;
-  }
-};
-
 // Streamed circuits whose plans differ only in coefficient values: their
 // states lie back to back in the pool and their packed plans back to back in
 // the plan buffer (table positions first .. first + count - 1), and each
@@ -175,11 +146,6 @@ struct sq_batch {
   uint32_t last_ctas = 0;
   const void *graph_fn = nullptr;
   bool last_jit = false;  // the last gradient run used the JIT kernel
-  // Plans of the gradient runs by structure, kept while the circuits are the
-  // same (angles may change): planning took 4 of the 7.8 ms of a run of 64 sets
-  // of a QAOA circuit (16 qubits, p = 8).
-  PlanShare grad_plans;
-  uint64_t grad_version = ~uint64_t(0);
   // Launch configuration (0 = default): tile bits, low bits of a streamed
   // tile, ops per sweep, CTAs per SM.
   uint32_t tile_bits = 0, low_bits = 0, max_ops = 0, ctas_per_sm = 0;
@@ -292,6 +258,36 @@ void pack_sweep(const sq::PlannedSweep &ps, std::vector<unsigned char> &out) {
 }
 
 // Plans one circuit into packed sweeps; returns the sweep count or < 0.
+// Plans shared between the circuits of one structure within one planning
+// pass (many parameter sets of one ansatz): the first circuit of a structure
+// (op signature, qubits, plan options) is planned, the others re-emit its
+// plan with their own values (sq::rebuild_plan), and fall back to planning
+// when that fails.
+struct PlanShare {
+  using Key = std::tuple<uint64_t, uint64_t, uint64_t, uint32_t>;
+  std::mutex mu;
+  std::map<Key, std::shared_ptr<const std::vector<sq::PlannedLaunch>>> plans;
+
+  std::vector<sq::PlannedLaunch> plan(const std::vector<sq::HostOp> &ops, uint32_t n, const sq::PlanOptions &opt) {
+    const auto sig = sq::op_signature_hash(ops);
+    const Key key{sig.first, sig.second, sq::plan_options_key(opt), n};
+    std::shared_ptr<const std::vector<sq::PlannedLaunch>> have;
+    {
+      std::lock_guard<std::mutex> lk(mu);
+      auto it = plans.find(key);
+      if (it != plans.end()) have = it->second;
+    }
+    if (have) {
+      std::vector<sq::PlannedLaunch> p = *have;
+      if (sq::rebuild_plan(p, ops, n)) return p;
+    }
+    std::vector<sq::PlannedLaunch> p = sq::plan_sweeps(ops, n, opt);
+    std::lock_guard<std::mutex> lk(mu);
+    plans.emplace(key, std::make_shared<const std::vector<sq::PlannedLaunch>>(p));
+    return p;
+  }
+};
+
 // A circuit's gates as planner ops (identities dropped).  False with `err`.
 bool circuit_host_ops(const Circ &c, std::vector<sq::HostOp> &ops, std::string &err) {
   ops.clear();
@@ -1085,12 +1081,8 @@ int run_gradient_impl(sq_batch *b, uint32_t n_params, double *energies, double *
   // the kernel that runs one circuit per CTA.
   bool try_multi = multi_enabled() && b->circs[0].n > M && b->circs[0].n >= sq::kApplyBits;
   for (size_t i = 1; i < nc; ++i) try_multi = try_multi && b->circs[i].n == b->circs[0].n;
-  if (b->grad_version != b->version) {
-    b->grad_plans.plans.clear();
-    b->grad_version = b->version;
-  }
   auto plan_all = [&](bool as_multi) {
-    PlanShare &share = b->grad_plans;
+    PlanShare share;
     next = 0;
     std::vector<std::thread> workers;
     for (unsigned t = 0; t < nth; ++t)
