@@ -799,7 +799,7 @@ int run_impl(sq_batch *b, double *energies, cudaStream_t st) {
     G.pool_off = tab[G.first].state_off;
     G.plan_off = tab[G.first].plan_off;
   }
-  // Work items of the energy pass: (pass, tile) of every deferred circuit.
+  // Work items of the energy pass: chunks of (pass, tile) of every deferred circuit.
   // Staged as [deferred | item_off (ndef+1)]; the kernel finds an item's
   // circuit by binary search over item_off.
   {
@@ -809,7 +809,8 @@ int run_impl(sq_batch *b, double *energies, cudaStream_t st) {
       const sq::BatchCircuit &t = tab[b->deferred[k]];
       const sq::PauliTilePlan &T = b->ham_tiles[t.ham];
       if (T.m != sq::kPauliTileBits) return fail(SQ_ERR_INVALID, "internal: a streamed state below one energy tile");
-      item_off.push_back(item_off.back() + (T.npasses << (T.n - T.m)));
+      item_off.push_back(item_off.back() +
+                         ((T.npasses << (T.n - T.m)) + sq::kEnergyTiles - 1) / sq::kEnergyTiles);
       b->tile_terms = std::max(b->tile_terms, T.max_terms);
       b->tile_groups = std::max(b->tile_groups, T.max_groups);
     }

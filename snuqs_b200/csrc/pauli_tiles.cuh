@@ -15,8 +15,7 @@
 // on B200: 64 random strings (8 passes) and 25 diagonal ones on 25 qubits
 // complex128 1187 us together, with one read of the state per mask 6212 us;
 // 2110 us with per-row sign flips and own amplitudes chosen at run time, 1670
-// us with a group header and a term loop for every single string.  The energy
-// pass of 512 VQE circuits of 8..20 qubits: 4.0 ms, before 11.9 ms.
+// us with a group header and a term loop for every single string.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
