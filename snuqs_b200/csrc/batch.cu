@@ -483,10 +483,12 @@ uint32_t batch_default_bits() {
 
 // Low index bits of the tiles of multi-state sweeps: runs of 128 bytes, as a
 // flush plans (512 VQE circuits of 8..20 qubits complex128: 47 sweeps in 7.65
-// ms; with the planner's 512-byte runs 57 in 7.93 ms).
+// ms; with the planner's 512-byte runs 57 in 7.93 ms).  complex64 keeps the
+// planner's: another plan is another order of FP32 roundings, which the FP64
+// energies show.
 template <typename Real>
 uint32_t multi_low_bits(uint32_t n) {
-  return sq::auto_low_bits(sizeof(Real) == 4, n, batch_default_bits<Real>());
+  return sizeof(Real) == 4 ? 0 : sq::auto_low_bits(false, n, batch_default_bits<Real>());
 }
 
 template <typename Real>
@@ -985,9 +987,9 @@ bool plan_gradient_circuit(const Circ &c, uint32_t m, std::vector<unsigned char>
     ropt.max_dense_k = sq::kAdjRegBits;
     if (multi) {
       // Multi-state sweeps: the tiles of the single-state passes.
-      ropt.tile_bits = uint32_t(sizeof(Real) == 4 ? sq::kAdjTileBitsC64[2] : sq::kAdjTileBitsC128[2]);
+      ropt.tile_bits = uint32_t(sq::kAdjTileBitsC128[2]);
       fopt.tile_bits = batch_default_bits<Real>();
-      fopt.low_bits = sq::auto_low_bits(sizeof(Real) == 4, c.n, fopt.tile_bits);
+      fopt.low_bits = multi_low_bits<Real>(c.n);
       fopt.select = ropt.select = multi_select();
     }
     const auto fplan = share ? share->plan(ap.forward, c.n, fopt) : sq::plan_sweeps(ap.forward, c.n, fopt);
@@ -1119,10 +1121,13 @@ int run_gradient_impl(sq_batch *b, uint32_t n_params, double *energies, double *
   std::vector<char> ok(nc, 0);
   std::atomic<size_t> next{0};
   const unsigned nth = std::max(1u, std::min(16u, std::thread::hardware_concurrency()));
-  // Circuits of one size above the tile are planned for multi-state sweeps
-  // (parameter sets of one circuit); when their plans turn out to differ, for
-  // the kernel that runs one circuit per CTA.
-  bool try_multi = multi_enabled() && b->circs[0].n > M && b->circs[0].n >= sq::kApplyBits;
+  // complex128 circuits of one size above the tile are planned for multi-state
+  // sweeps (parameter sets of one circuit); when their plans turn out to
+  // differ, for the kernel that runs one circuit per CTA.  complex64 stays
+  // with that kernel: the multi-state reverse sweeps take smaller tiles, and
+  // another plan is another order of FP32 roundings, which the FP64 gradients
+  // show.
+  bool try_multi = sizeof(Real) == 8 && multi_enabled() && b->circs[0].n > M && b->circs[0].n >= sq::kApplyBits;
   for (size_t i = 1; i < nc; ++i) try_multi = try_multi && b->circs[i].n == b->circs[0].n;
   auto plan_all = [&](bool as_multi) {
     PlanShare share;

@@ -1286,9 +1286,11 @@ int adjoint_impl(sq_state *psi, sq_state *lam, const sq::AdjointPlan &ap, const 
   fopt.tile_bits = pick_tile_bits(psi->dtype, n, psi->tile_bits);
   fopt.max_dense_k = sizeof(Real) == 4 ? 4 : 3;
   // 128-byte runs, as a flush plans: 12 forward sweeps instead of 15 (QAOA
-  // p = 8, 24 qubits complex128: 2.20 instead of 2.38 ms).  The reverse sweeps
-  // keep the longer runs: bound by FP64, 16 to 20 of them take the same time.
-  fopt.low_bits = sq::auto_low_bits(sizeof(Real) == 4, n, fopt.tile_bits);
+  // p = 8, 24 qubits complex128: 2.20 instead of 2.38 ms).  complex64 keeps the
+  // longer runs: another plan is another order of FP32 roundings, which its
+  // FP64 results show.  The reverse sweeps keep them too: bound by FP64, 16 to
+  // 20 of them take the same time.
+  if (sizeof(Real) == 8) fopt.low_bits = sq::auto_low_bits(false, n, fopt.tile_bits);
   std::vector<sq::PlannedLaunch> fplan, rplan;
   sq::PlanOptions ropt;
   ropt.tile_bits = pick_adjoint_tile_bits(psi->dtype, n);

@@ -397,6 +397,31 @@ std::string inner_call(const SweepOp &op, const char *R, const std::string &bits
   return s.str();
 }
 
+// The same with both parts of the complex product, into doubles sr, si: the
+// complex64 batched-gradient kernel.  Its compiled FP32 roundings (which of two
+// products an FMA takes) follow the code around them, and with the real-part
+// form its gradients were 8.5e-9 from those of this one.
+std::string inner_call_both(const SweepOp &op, const char *R, const std::string &bits) {
+  std::ostringstream s;
+  const bool pauli = op.aux & kAuxPauli;
+  if (op.kind == kSwInnerDiag) {
+    s << bits << " ";
+    if (pauli)
+      s << "inner_diag_pauli<" << R << ", " << int(op.vmask) << ", " << int(op.aux & 7) << ">";
+    else
+      s << "inner_diag<" << R << ", " << int(op.vmask) << ">";
+    s << "(F, G, coef + " << op.coef << ", b, sr, si); ";
+  } else {
+    if (pauli)
+      s << "inner_dense_pauli<" << R << ", " << int(op.vmask) << ", " << int(op.aux & 7) << ", "
+        << int((op.aux >> 3) & 7) << ">";
+    else
+      s << "inner_dense<" << R << ", " << int(op.vmask) << ">";
+    s << "(F, G, coef + " << op.coef << ", sr, si); ";
+  }
+  return s.str();
+}
+
 // Fused code for a run of consecutive diagonal ops of one phase (kSwDiag,
 // kSwPhase): instead of one complex multiply per amplitude per op, the run's
 // factors are multiplied together first and applied once.  Each op's factor
@@ -646,10 +671,15 @@ void one_state_ops_src(const SweepOp *ops, const SweepPhase &ph, const char *R, 
 // Pauli-Z ones from one shared set of products conj(lambda_r) phi_r; then
 // the run's diagonal ops, fused, on both states.  False when an op is not
 // covered (an inner product with conditions).
-bool two_state_ops_src(const SweepOp *ops, const SweepPhase &ph, const char *R, bool c64, int NT, std::ostream &s) {
+bool two_state_ops_src(const SweepOp *ops, const SweepPhase &ph, const char *R, bool c64, int NT, std::ostream &s,
+                       bool both_parts = false) {
   auto cf = [](const SweepOp &o) { return "(coef + " + std::to_string(o.coef) + ")"; };
   auto inner_plain = [&](const SweepOp &op) {
-    s << "      { " << inner_call(op, R, diag_bits_src(op), NT) << " }\n";
+    if (both_parts)
+      s << "      { double sr = 0.0, si = 0.0; " << inner_call_both(op, R, diag_bits_src(op)) << "jit_inner_acc<" << NT
+        << ", " << op.slot << ">(acc, sr, si); }\n";
+    else
+      s << "      { " << inner_call(op, R, diag_bits_src(op), NT) << " }\n";
   };
   auto single = [&](const SweepOp &op) {
     std::string tmpl;
@@ -687,7 +717,29 @@ bool two_state_ops_src(const SweepOp *ops, const SweepPhase &ph, const char *R, 
       else
         diag.push_back(&op);
     }
-    if (!pauli.empty()) {
+    if (!pauli.empty() && both_parts) {
+      s << "      { // " << pauli.size() << " Pauli-Z inner products from shared products\n";
+      for (int ri = 0; ri < kAdjAmps; ++ri)
+        s << "        const double p" << ri << "r = fma(double(G.re[" << ri << "]), double(F.re[" << ri
+          << "]), double(G.im[" << ri << "]) * double(F.im[" << ri << "])), p" << ri << "i = fma(double(G.re["
+          << ri << "]), double(F.im[" << ri << "]), -double(G.im[" << ri << "]) * double(F.re[" << ri << "]));\n";
+      for (const SweepOp *op : pauli) {
+        const int V = op->vmask, Z = op->aux & 7, nv = __builtin_popcount(uint32_t(V));
+        std::ostringstream qr, qi;
+        for (int ri = 0; ri < kAdjAmps; ++ri) {
+          const bool neg = __builtin_popcount(uint32_t(bit_ext(ri, V) & Z)) & 1;
+          qr << (neg ? " - " : " + ") << "p" << ri << "r";
+          qi << (neg ? " - " : " + ") << "p" << ri << "i";
+        }
+        s << "        { double qr = 0.0" << qr.str() << ", qi = 0.0" << qi.str() << ";";
+        if (Z >> nv)
+          s << " " << diag_bits_src(*op) << " if (__popc(b & " << (Z >> nv) << "u) & 1) { qr = -qr; qi = -qi; }";
+        s << "\n          const auto a = " << cf(*op) << "[0];\n"
+          << "          jit_inner_acc<" << NT << ", " << op->slot << ">(acc, double(a.x) * qr - double(a.y) * qi, "
+          << "double(a.x) * qi + double(a.y) * qr); }\n";
+      }
+      s << "      }\n";
+    } else if (!pauli.empty()) {
       // Im conj(lambda_r) phi_r once per amplitude (alpha is imaginary, so the
       // gradient needs no more), and its sums under the eight sign patterns
       // of the register bits by a Walsh transform (24 additions); an op is
@@ -999,7 +1051,7 @@ std::string jit_batch_adjoint_body(const unsigned char *plan, uint32_t nfwd, uin
       fns << "  jit_batch_fwd<" << R << ", " << M << ", Tile>(psi, bufs, " << ps.h.num_tiles
           << "ull, [&](C2 *tile, uint64_t gbase) {\n";
     else
-      fns << " " << inner_slots(ops, ps.nops, false, NT) << "\n  jit_batch_rev<" << R << ", " << M << ", Tile>(psi, lam, bufs, " << ps.h.num_tiles
+      fns << " " << (c64 ? "" : inner_slots(ops, ps.nops, false, NT)) << "\n  jit_batch_rev<" << R << ", " << M << ", Tile>(psi, lam, bufs, " << ps.h.num_tiles
           << "ull, [&](C2 *ft, C2 *lt, uint64_t gbase) {\n";
     for (uint32_t p = 0; p < ps.h.nphases; ++p) {
       const SweepPhase &P = ph[p];
@@ -1021,12 +1073,12 @@ std::string jit_batch_adjoint_body(const unsigned char *plan, uint32_t nfwd, uin
         for (int t : thread_positions(P, int(M), c64, false, kAdjRegBits)) fns << ", " << t;
         fns << ">;\n      const uint32_t jb = Ph::jb(threadIdx.x);\n      Amps<" << R << ", " << kAdjAmps
             << "> F, G;\n      Ph::gather(F, G, ft, lt, jb);\n";
-        if (!two_state_ops_src(ops, P, R, c64, NT, fns)) return std::string();
+        if (!two_state_ops_src(ops, P, R, c64, NT, fns, c64)) return std::string();
         fns << "      Ph::scatter(F, G, ft, lt, jb);\n      __syncthreads(); }\n";
       }
     }
     fns << "  });\n";
-    if (rev) fns << " " << inner_slots(ops, ps.nops, true, NT) << "\n  __syncthreads();\n";
+    if (rev && !c64) fns << " " << inner_slots(ops, ps.nops, true, NT) << "\n  __syncthreads();\n";
     if (rev && inner) {
       fns << "  if (threadIdx.x == 0) {\n";
       for (uint32_t q = 0; q < inner[0]; ++q)

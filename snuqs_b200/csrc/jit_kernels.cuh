@@ -43,12 +43,11 @@ __device__ __forceinline__ void jit_cmul_acc(Real &ar, Real &ai, Real br, Real b
 }
 
 // op_dense with all rows of a group advancing together over the columns (the
-// same sums, left to right over the columns): 2 * 2^k independent chains
-// instead of two.  complex64 matrices of one and two
+// same sums, left to right over the columns: the same bits): 2 * 2^k
+// independent chains instead of two.  complex64 matrices of one and two
 // qubits, whose coefficients are constant-bank operands, so that nothing but
 // the chains' latency is between the FMAs: volume circuits of 27 qubits on
-// B200 spend 6 % less in their sweeps (33.5 -> 31.6 ms for depth 27; error of
-// 25-qubit states against complex128 1.03e-6 both ways).  complex128
+// B200 spend 6 % less in their sweeps (33.5 -> 31.6 ms for depth 27).  complex128
 // is bound by the FP64 pipe either way (10.2 ms both for depth 8 at 26 qubits).
 template <typename Real, int NA, int V, class CP>
 __device__ __forceinline__ void jit_op_dense(Amps<Real, NA> &A, CP c, int rmask, int rval) {
@@ -61,10 +60,15 @@ __device__ __forceinline__ void jit_op_dense(Amps<Real, NA> &A, CP c, int rmask,
 #pragma unroll
       for (int r = 0; r < D; ++r) {
         const auto m = c[r * D + x];
-        sr[r] = x ? fma(m.x, ar, sr[r]) : m.x * ar;
-        si[r] = x ? fma(m.x, ai, si[r]) : m.x * ai;
-        sr[r] = fma(-m.y, ai, sr[r]);
-        si[r] = fma(m.y, ar, si[r]);
+        if (x == 0) {  // the roundings the compiler gives op_dense's first column
+          sr[r] = fma(m.x, ar, -(m.y * ai));
+          si[r] = fma(m.y, ar, m.x * ai);
+        } else {
+          sr[r] = fma(m.x, ar, sr[r]);
+          sr[r] = fma(-m.y, ai, sr[r]);
+          si[r] = fma(m.x, ai, si[r]);
+          si[r] = fma(m.y, ar, si[r]);
+        }
       }
     }
 #pragma unroll
@@ -759,6 +763,22 @@ __device__ __forceinline__ double real_inner_diag_pauli(const Amps<Real, kAdjAmp
   }
   const double q = (__popc(b & uint32_t(Z >> ct_popc<V>())) & 1) ? p - m : m - p;
   return double(c[0].y) * q;
+}
+
+// Both parts (complex64 batched-gradient kernel).
+template <int NT, int SLOT>
+__device__ __forceinline__ void jit_inner_acc(double2 *acc, double sr, double si) {
+  constexpr unsigned kMask = NT >= 32 ? 0xffffffffu : ((1u << NT) - 1u);
+#pragma unroll
+  for (int off = (NT >= 32 ? 16 : NT / 2); off > 0; off >>= 1) {
+    sr += __shfl_xor_sync(kMask, sr, off);
+    si += __shfl_xor_sync(kMask, si, off);
+  }
+  if ((threadIdx.x & 31) == 0) {
+    double2 &a = acc[(threadIdx.x >> 5) * kMaxInner + SLOT];
+    a.x += sr;
+    a.y += si;
+  }
 }
 
 // Adds one thread's share of slot SLOT to its warp's sum (warp shuffles, then

@@ -23,28 +23,13 @@ namespace {
 
 int popc64(uint64_t x) { return __builtin_popcountll(x); }
 
-// The distinct inner-product slots of a sweep (at most kMaxInner).
-struct InnerSlotSet {
-  uint32_t slot[kMaxInner], count = 0;
-  bool has(uint32_t s) const {
-    for (uint32_t i = 0; i < count; ++i)
-      if (slot[i] == s) return true;
-    return false;
-  }
-  bool fits(uint32_t s) const { return count < uint32_t(kMaxInner) || has(s); }
-  void add(uint32_t s) {
-    if (!has(s)) slot[count++] = s;
-  }
-};
-
 struct SweepBuilder {
   uint32_t n, m, l, max_dense_k = 3, reg_bits = kRegBits, max_ops = kMaxOps;
   uint64_t S;  // tile bits (global index bits)
   std::vector<const HostOp *> ops;
   std::vector<uint64_t> phase_regs;  // register bits (global) of each phase
   std::vector<uint32_t> phase_first; // first op index of each phase
-  uint32_t ncoef = 0;
-  InnerSlotSet inner;
+  uint32_t ncoef = 0, ninner = 0;
   // Remap: output global bit of the content of every global bit (size n;
   // empty = the identity).  Only tile bits move.
   std::vector<int> outmap;
@@ -64,7 +49,7 @@ struct SweepBuilder {
   bool try_add(const HostOp &op) {
     if (ops.size() >= size_t(max_ops)) return false;
     if (ncoef + coef_count(op) > uint32_t(kMaxCoef)) return false;
-    if (op.kind == kOpInner && !inner.fits(op.slot)) return false;
+    if (op.kind == kOpInner && ninner >= uint32_t(kMaxInner)) return false;
     if (is_diag(op)) {
       if (op.tbits.size() > size_t(kMaxDiagK)) return false;
       if (phase_regs.empty()) {
@@ -73,7 +58,7 @@ struct SweepBuilder {
       }
       ops.push_back(&op);
       ncoef += coef_count(op);
-      if (op.kind == kOpInner) inner.add(op.slot);
+      if (op.kind == kOpInner) ++ninner;
       return true;
     }
     const uint32_t kmax = op.kind == kOpInner ? reg_bits : max_dense_k;
@@ -91,7 +76,7 @@ struct SweepBuilder {
     }
     ops.push_back(&op);
     ncoef += coef_count(op);
-    if (op.kind == kOpInner) inner.add(op.slot);
+    if (op.kind == kOpInner) ++ninner;
     return true;
   }
 
@@ -406,7 +391,7 @@ uint32_t op_budget(const PlanOptions &opt) {
 // that copy).
 struct OpInfo {
   uint64_t T, A, tm;  // non-diagonal, touched and target bits
-  uint32_t coef, slot;
+  uint32_t coef;
   bool diag, fits, inner;
 };
 
@@ -423,7 +408,6 @@ struct OpTable {
     f.diag = SweepBuilder::is_diag(op);
     f.fits = fusable_size(op, opt);
     f.inner = op.kind == kOpInner;
-    f.slot = op.slot;
   }
 };
 
@@ -431,8 +415,7 @@ struct OpTable {
 // the collection below, without growing S).
 uint32_t absorbed(const std::vector<const HostOp *> &rem, size_t head, uint64_t S, uint32_t n,
                   const PlanOptions &opt, size_t window, const OpTable &tab) {
-  uint32_t cnt = 0, ncoef = 0;
-  InnerSlotSet inner;
+  uint32_t cnt = 0, ncoef = 0, ninner = 0;
   const uint32_t max_ops = op_budget(opt);
   uint64_t blockT = 0, blockA = 0;
   size_t skipped = 0;
@@ -443,11 +426,11 @@ uint32_t absorbed(const std::vector<const HostOp *> &rem, size_t head, uint64_t 
     const bool diag = f.diag;
     const uint32_t c = f.coef;
     const bool fits = f.fits && (diag || (f.tm & ~S) == 0) && cnt < max_ops &&
-                      ncoef + c <= uint32_t(kMaxCoef) && !(f.inner && !inner.fits(f.slot));
+                      ncoef + c <= uint32_t(kMaxCoef) && !(f.inner && ninner >= uint32_t(kMaxInner));
     if (commutes && fits) {
       ++cnt;
       ncoef += c;
-      if (f.inner) inner.add(f.slot);
+      if (f.inner) ++ninner;
       if (cnt >= max_ops) break;
       continue;
     }
@@ -744,8 +727,7 @@ std::vector<PlannedLaunch> plan_sweeps(const std::vector<HostOp> &ops, uint32_t 
       std::vector<const HostOp *> chosen;
       std::vector<size_t> chosen_idx, skipped_idx;
       uint64_t blockT = 0, blockAll = 0;
-      uint32_t ncoef = 0;
-      InnerSlotSet inner;
+      uint32_t ncoef = 0, ninner = 0;
       size_t i = head;
       for (; i < rem.size(); ++i) {
         const HostOp &op = *rem[i];
@@ -756,13 +738,13 @@ std::vector<PlannedLaunch> plan_sweeps(const std::vector<HostOp> &ops, uint32_t 
         const uint32_t c = f.coef;
         const bool fits = f.fits && (diag || uint32_t(popc64(S | f.tm)) <= m) &&
                           chosen.size() < size_t(sb.max_ops) && ncoef + c <= uint32_t(kMaxCoef) &&
-                          !(f.inner && !inner.fits(f.slot));
+                          !(f.inner && ninner >= uint32_t(kMaxInner));
         if (commutes && fits) {
           if (!diag) S |= f.tm;
           chosen.push_back(&op);
           chosen_idx.push_back(i);
           ncoef += c;
-          if (f.inner) inner.add(f.slot);
+          if (f.inner) ++ninner;
           if (chosen.size() >= size_t(sb.max_ops)) {
             ++i;
             break;
@@ -811,7 +793,7 @@ std::vector<PlannedLaunch> plan_sweeps(const std::vector<HostOp> &ops, uint32_t 
       sb.ops = order;
       for (const HostOp *op : order) {
         sb.ncoef += SweepBuilder::coef_count(*op);
-        if (op->kind == kOpInner) sb.inner.add(op->slot);
+        if (op->kind == kOpInner) ++sb.ninner;
       }
       PlannedLaunch pl;
       pl.is_sweep = true;
@@ -941,7 +923,7 @@ bool rebuild_sweep(const SweepRecipe &r, const std::vector<HostOp> &ops, uint32_
     if (i >= ops.size()) return false;
     sb.ops.push_back(&ops[i]);
     sb.ncoef += SweepBuilder::coef_count(ops[i]);
-    if (ops[i].kind == kOpInner) sb.inner.add(ops[i].slot);
+    if (ops[i].kind == kOpInner) ++sb.ninner;
   }
   out = sb.finish();
   out.recipe = r;
