@@ -46,8 +46,8 @@ __device__ __forceinline__ void jit_cmul_acc(Real &ar, Real &ai, Real br, Real b
 // same sums, left to right over the columns: the same bits): 2 * 2^k
 // independent chains instead of two.  complex64 matrices of one and two
 // qubits, whose coefficients are constant-bank operands, so that nothing but
-// the chains' latency is between the FMAs: volume circuits of 27 qubits on
-// B200 spend 6 % less in their sweeps (33.5 -> 31.6 ms for depth 27).  complex128
+// the chains' latency is between the FMAs: the sweeps of a volume circuit of
+// 27 qubits and depth 27 take 32.5 instead of 33.7 ms on B200.  complex128
 // is bound by the FP64 pipe either way (10.2 ms both for depth 8 at 26 qubits).
 template <typename Real, int NA, int V, class CP>
 __device__ __forceinline__ void jit_op_dense(Amps<Real, NA> &A, CP c, int rmask, int rval) {
