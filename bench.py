@@ -197,6 +197,10 @@ def run_reference(args, rank, world):
         return
     import oracle
 
+    if not oracle.ref_available():
+        print(json.dumps({"impl": "reference", "unavailable":
+                          "the reference's sources are not here to build its CPU gate path from"}))
+        return
     n, ops = args.qubits, pseudo_sorted(circuit(args.qubits, args.gates))
     if not host_ram_ok(n):
         print(json.dumps({"impl": "reference", "unavailable":

@@ -193,9 +193,12 @@ int oracle_apply(double *state, int nq, const double *matrix,
     off[c] = o;
   }
   for (int j = 0; j < k; ++j) tmask |= (uint64_t)1 << (nq - 1 - targets[j]);
-  cplx a[1024];
+  /* The groups are independent of each other (as the reference's own loop,
+   * which OpenMP splits): every group's arithmetic is the same on any thread. */
+#pragma omp parallel for if (nq >= 16)
   for (uint64_t i = 0; i < n; ++i) {
     if (i & tmask) continue;
+    cplx a[1024];
     for (int c = 0; c < d; ++c) a[c] = psi[i + off[c]];
     for (int r = 0; r < d; ++r) {
       cplx acc = cmul(g[r * d], a[0]);
