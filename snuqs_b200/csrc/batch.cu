@@ -592,6 +592,8 @@ int run_impl(sq_batch *b, double *energies, cudaStream_t st) {
   const uint32_t M = batch_tile_bits<Real>(b);
   const size_t nc = b->circs.size();
   if (nc == 0) return SQ_OK;
+  // Kernel attributes and occupancy are the current device's, so before any of them.
+  SQB_CUDA(cudaSetDevice(b->device));
   const void *fn = nullptr;
   int threads = 0, per_sm = 0;
   size_t smem = 0;
@@ -769,7 +771,6 @@ int run_impl(sq_batch *b, double *energies, cudaStream_t st) {
   }
   plan_bytes = 0;
   for (size_t i = 0; i < nc; ++i) plan_bytes += packed[i].size();
-  SQB_CUDA(cudaSetDevice(b->device));
   if (int s = b->d_pool.ensure(std::max<uint64_t>(pool_amps, 1) * sizeof(C2))) return s;
   if (int s = b->d_plans.ensure(plan_bytes + 16)) return s;
   if (int s = b->h_plans.ensure(plan_bytes + 16)) return s;
@@ -1108,6 +1109,7 @@ int run_gradient_impl(sq_batch *b, uint32_t n_params, double *energies, double *
   const uint32_t M = batch_adj_fn<Real>(b->tile_bits) ? b->tile_bits : batch_default_bits<Real>();
   const size_t nc = b->circs.size();
   if (nc == 0) return SQ_OK;
+  SQB_CUDA(cudaSetDevice(b->device));  // before any kernel attribute or occupancy, as in run_impl
   // This run restages the shared buffers: the energy run's plan cache and
   // graph are no longer valid.
   b->planned_version = ~uint64_t(0);
@@ -1216,7 +1218,6 @@ int run_gradient_impl(sq_batch *b, uint32_t n_params, double *energies, double *
   if (try_multi) pool_amps *= 2;
   size_t plan_bytes = 0;
   for (size_t i = 0; i < nc; ++i) plan_bytes += packed[i].size();
-  SQB_CUDA(cudaSetDevice(b->device));
   if (int s = b->d_pool.ensure(std::max<uint64_t>(pool_amps, 1) * sizeof(C2))) return s;
   if (int s = b->d_plans.ensure(plan_bytes + 16)) return s;
   if (int s = b->h_plans.ensure(plan_bytes + 16)) return s;
@@ -1544,6 +1545,7 @@ int sq_batch_run(sq_batch *b, double *energies, void *stream) {
 int sq_batch_autotune(sq_batch *b, uint32_t reps, sq_batch_config *best, void *stream) {
   if (!b) return fail(SQ_ERR_INVALID, "null batch");
   if (b->circs.empty()) return fail(SQ_ERR_INVALID, "batch autotune: no circuits");
+  SQB_CUDA(cudaSetDevice(b->device));
   auto st = static_cast<cudaStream_t>(stream);
   reps = std::max<uint32_t>(1, std::min<uint32_t>(reps, 16));
   std::vector<double> e(b->circs.size());

@@ -18,5 +18,16 @@ def build() -> str:
     return OUT
 
 
+def build_fake(folder: str) -> str:
+    """In `folder`: the engine's objects (left by snuqs_b200.build) linked with
+    fake_cudart.cc in place of the CUDA runtime."""
+    out, objs = os.path.join(folder, "libsnuqs_fake_cuda.so"), os.path.join(os.path.dirname(CSRC), "_build")
+    subprocess.run(["g++", "-O1", "-std=c++17", "-fPIC", "-shared", "-I", "/usr/local/cuda/include",
+                    os.path.join(HERE, "fake_cudart.cc"),
+                    *sorted(os.path.join(objs, f) for f in os.listdir(objs) if f.endswith(".o")),
+                    "-o", out, "-ldl", "-lpthread", "-Wl,--no-undefined", "-Wl,-Bsymbolic"], check=True)
+    return out
+
+
 if __name__ == "__main__":
     print(build())
