@@ -870,7 +870,7 @@ int run_impl(sq_batch *b, double *energies, cudaStream_t st) {
   if (esmem > 48 * 1024)
     SQB_CUDA(cudaFuncSetAttribute(sq::batch_energy_tiles<Real>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   int(sq::pauli_tile_smem(sq::kPauliMaxTerms, sq::kPauliMaxGroups))));
-  if (int s = b->d_part.ensure(std::max<size_t>(b->nitems, 1) * sizeof(double))) return s;
+  if (int s = b->d_part.ensure(std::max<size_t>(b->nitems, 1) * 2 * sizeof(double))) return s;
   // (Re)capture the graph when sizes or the stream changed.
   if (!b->graph || b->graph_plan_bytes != plan_bytes || b->graph_ncirc != nc ||
       b->graph_stream != st || b->graph_grid != grid || b->graph_fn != fn) {
@@ -940,7 +940,7 @@ int run_impl(sq_batch *b, double *energies, cudaStream_t st) {
         sq::batch_energy_tiles<Real><<<egrid, sq::kPauliThreads, esmem, cs>>>(
             poolp, P.circuits, static_cast<const sq::PauliTilePlan *>(b->d_tiles.p), defp, offp, ndef, b->nitems,
             b->tile_terms, partp);
-        sq::batch_energy_finalize<<<ndef, sq::kReduceThreads, 0, cs>>>(partp, offp, defp, P.energies);
+        sq::batch_energy_finalize<<<ndef, sq::kReduceThreads, 0, cs>>>(partp, offp, b->nitems, defp, P.energies);
       }
       cudaEventRecordWithFlags(b->ev1, cs, cudaEventRecordExternal);
       cudaMemcpyAsync(b->h_energy.p, b->d_energy.p, nc * sizeof(double), cudaMemcpyDeviceToHost, cs);

@@ -2,9 +2,9 @@
 // sweeps: the tiled Pauli expectation (pauli_tiles.cuh) over work items of all
 // of them.  Deferred circuit k has passes(Hamiltonian) x 2^(n - m) tiles to
 // work, pass by pass, in chunks of kEnergyTiles; its chunks are numbered from
-// chunk_off[k].  partials[w] receives the sum of chunk w, and
-// batch_energy_finalize adds a circuit's chunks in order (the sums do not
-// depend on the grid).
+// chunk_off[k].  partials[w], partials[nchunks + w] receive the carried sum of
+// chunk w, and batch_energy_finalize adds a circuit's chunks in order (the sums
+// do not depend on the grid).
 //
 // Bound: shared-memory reads (pauli_tiles.cuh); the states come from L2 (the
 // chunks running at any one time belong to a few neighbouring circuits), once
@@ -42,16 +42,32 @@ __global__ void __launch_bounds__(kPauliThreads, 4)
     const uint32_t first = (w - chunk_off[k]) * kEnergyTiles;
     const uint32_t last = first + kEnergyTiles < items ? first + kEnergyTiles : items;
     uint32_t staged = ~0u;
-    double s = 0.0;
+    CarriedSum acc{0.0, 0.0};
     for (uint32_t j = first; j < last; ++j) {
       const uint32_t pass = j >> tile_bits;
       if (pass != staged) pauli_stage(T, T.pass[pass], sh);
       staged = pass;
-      s += pauli_tile<Real, true>(psi, T, T.pass[pass], j & ((1u << tile_bits) - 1u), sh);
+      carry_add(acc, pauli_tile<Real, true>(psi, T, T.pass[pass], j & ((1u << tile_bits) - 1u), sh), 0.0);
     }
-    s = block_sum(s);
-    if (threadIdx.x == 0) partials[w] = s;
+    const CarriedSum s = block_sum(acc);
+    if (threadIdx.x == 0) {
+      partials[w] = s.hi;
+      partials[nchunks + w] = s.lo;
+    }
   }
+}
+
+// energies[deferred[k]] = sum of the chunks [chunk_off[k], chunk_off[k + 1]), in
+// order.  One block per deferred circuit.
+static __global__ void __launch_bounds__(kReduceThreads)
+    batch_energy_finalize(const double *__restrict__ partials, const uint32_t *__restrict__ chunk_off,
+                          uint32_t nchunks, const uint32_t *__restrict__ deferred, double *__restrict__ energies) {
+  const uint32_t k = blockIdx.x;
+  CarriedSum v{0.0, 0.0};
+  for (uint32_t i = chunk_off[k] + threadIdx.x; i < chunk_off[k + 1]; i += blockDim.x)
+    carry_add(v, partials[i], partials[nchunks + i]);
+  v = block_sum(v);
+  if (threadIdx.x == 0) energies[deferred[k]] = carried(v);
 }
 
 }  // namespace sq

@@ -227,17 +227,6 @@ __global__ void __launch_bounds__(1 << (M - kRegBits), 1)
 }
 
 // Streamed (pool-resident) circuits leave their energies to batch_energy.cuh.
-// energies[deferred[k]] = sum of partials[item_off[k] .. item_off[k+1]), in
-// order.  One block per deferred circuit.
-static __global__ void __launch_bounds__(kReduceThreads)
-    batch_energy_finalize(const double *__restrict__ partials, const uint32_t *__restrict__ item_off,
-                          const uint32_t *__restrict__ deferred, double *__restrict__ energies) {
-  const uint32_t k = blockIdx.x;
-  double v = 0.0;
-  for (uint32_t i = item_off[k] + threadIdx.x; i < item_off[k + 1]; i += blockDim.x) v += partials[i];
-  v = block_sum(v);
-  if (threadIdx.x == 0) energies[deferred[k]] = v;
-}
 
 // |0...0> in each of the K states of 2^n amplitudes that lie back to back
 // from psi (a structure group of a batch, before its multi-state sweeps);

@@ -1011,7 +1011,7 @@ static int expect_impl(sq_state *s, const std::vector<uint64_t> &xm,
     return (ny[a] & 1) < (ny[b] & 1);
   });
   const uint32_t blocks = uint32_t(di.sms) * 4;  // the kernel's resident blocks
-  SQ_TRY(ensure_scratch(s, blocks + 1));
+  SQ_TRY(ensure_scratch(s, 2 * blocks + 1));
   auto P = std::make_unique<sq::PauliTilePlan>();
   const uint32_t nterms = uint32_t(idx.size());
   uint32_t pos = 0;
@@ -1027,9 +1027,9 @@ static int expect_impl(sq_state *s, const std::vector<uint64_t> &xm,
                 : sq::launch_pauli_tiles<double>(s->data, *P, s->scratch, blocks, !first_launch, st));
     first_launch = false;
   }
-  sq::finalize_sum_kernel<<<1, sq::kReduceThreads, 0, st>>>(s->scratch, blocks, s->scratch + blocks);
+  sq::finalize_carried_kernel<<<1, sq::kReduceThreads, 0, st>>>(s->scratch, blocks, s->scratch + 2 * blocks);
   SQ_CUDA(cudaGetLastError());
-  SQ_CUDA(cudaMemcpyAsync(out, s->scratch + blocks, sizeof(double), cudaMemcpyDeviceToHost, st));
+  SQ_CUDA(cudaMemcpyAsync(out, s->scratch + 2 * blocks, sizeof(double), cudaMemcpyDeviceToHost, st));
   SQ_CUDA(cudaStreamSynchronize(st));
   return take_kernel_error(s);
 }

@@ -19,7 +19,7 @@
 // device share the array, so calls that overlap on the GPU race: order them
 // on one stream or with events.
 //
-// The array's limits: at most kNoAllocMaxBlocks (2048) reduction blocks
+// The array's limits: at most kNoAllocMaxBlocks (1024) reduction blocks
 // (16 KiB of FP64 partials), at most 1024 Pauli terms and 256 distinct
 // (X/Y mask, Y parity) groups per call.  Larger requests are rejected.
 // Each call stages the grouped terms on the calling thread's stack (about
@@ -38,11 +38,11 @@ int sq_detail_fail(int code, const char *msg);  // engine.cu: sets sq_last_error
 
 namespace {
 
-constexpr uint32_t kNoAllocMaxBlocks = 2048;
+constexpr uint32_t kNoAllocMaxBlocks = 1024;
 constexpr int kMaxDevices = 64;
 
 // Shared by every call on a device; each call overwrites the slots it uses.
-static __device__ __align__(256) double g_noalloc_partials[kNoAllocMaxBlocks];
+static __device__ __align__(256) double g_noalloc_partials[2 * kNoAllocMaxBlocks];
 
 std::mutex g_mu;
 double *g_partials_ptr[kMaxDevices] = {};
@@ -148,7 +148,7 @@ extern "C" int sq_expect_pauli_noalloc(const void *state, uint32_t num_qubits, i
   if (groups > sq::kPauliMaxGroups)
     return fail(SQ_ERR_UNSUPPORTED,
                 "sq_expect_pauli_noalloc: more than 256 distinct Pauli groups");
-  const uint32_t blocks = std::min(uint32_t(sms) * 4, uint32_t(kNoAllocMaxBlocks));
+  const uint32_t blocks = std::min(uint32_t(sms) * 4, kNoAllocMaxBlocks);
   sq::PauliTilePlan P;  // 26 KiB on the stack
   if (sq::plan_pauli_tiles(P, n, idx, n_terms, 0, xm, zym, ny, weights, blocks) != n_terms)
     return fail(SQ_ERR_UNSUPPORTED, "sq_expect_pauli_noalloc: the terms do not fit one plan");
@@ -159,7 +159,7 @@ extern "C" int sq_expect_pauli_noalloc(const void *state, uint32_t num_qubits, i
                       : sq::launch_pauli_tiles<double>(state, P, partials, blocks, 0, s);
   if (e != cudaSuccess) return fail(SQ_ERR_CUDA, cudaGetErrorString(e));
   // Fixed-order sum of the partials into the caller's output (deterministic).
-  sq::finalize_sum_kernel<<<1, sq::kReduceThreads, 0, s>>>(partials, blocks, out_device);
+  sq::finalize_carried_kernel<<<1, sq::kReduceThreads, 0, s>>>(partials, blocks, out_device);
   e = cudaGetLastError();
   if (e != cudaSuccess) return fail(SQ_ERR_CUDA, cudaGetErrorString(e));
   return SQ_OK;

@@ -1,0 +1,44 @@
+"""Rounding of sums of Pauli strings over whole states."""
+import numpy as np
+import pytest
+
+from snuqs_b200 import capi
+
+pytestmark = pytest.mark.gpu
+
+
+def ring(n):
+    return [(1.0, "".join("Z" if q in (i, (i + 1) % n) else "I" for q in range(n))) for i in range(n)]
+
+
+def exact_ring(psi, n):
+    """The same sum with x87 extended products and a compensated total."""
+    idx = np.arange(1 << n, dtype=np.uint64)
+    w = np.zeros(1 << n, dtype=np.int64)
+    for i in range(n):
+        a, b = np.uint64(n - 1 - i), np.uint64(n - 1 - (i + 1) % n)
+        w += 1 - 2 * (((idx >> a) ^ (idx >> b)) & np.uint64(1)).astype(np.int64)
+    re, im = psi.real.astype(np.longdouble), psi.imag.astype(np.longdouble)
+    return np.sum((re * re + im * im) * w)
+
+
+@pytest.mark.parametrize("n", [18, 19, 20, 21])
+def test_ring_sum_rounding(n):
+    """The ring sum of Z Z strings on random states cancels to about 2^-(n/2)
+    of its weights.  What a sum that carries its additions' errors leaves is
+    the rounding of the products: about a dozen roundings (eight rows, their
+    signed sums, the weights) of size 2^-53 * n * 2^-n for each of the 2^n
+    amplitudes, independent of each other, so 2^-53 * n * 2^-(n/2) times the
+    root of a dozen over the states; partial sums added plainly leave about
+    ten times that."""
+    rng = np.random.default_rng(n)
+    errors = []
+    for _ in range(12):
+        psi = rng.standard_normal(1 << n) + 1j * rng.standard_normal(1 << n)
+        psi /= np.linalg.norm(psi)
+        st = capi.State(n, capi.SQ_C128)
+        st.from_host(psi)
+        errors.append(float(np.longdouble(st.expectation(ring(n))) - exact_ring(psi, n)))
+        st.close()
+    rms = float(np.sqrt(np.mean(np.square(errors))))
+    assert rms <= 4.0 * 2.0 ** -53 * n * 2.0 ** (-n / 2), rms
