@@ -265,7 +265,7 @@ __device__ __forceinline__ double pauli_tile(const typename Vec2<Real>::T *__res
     sh.term[i].word = T.zt[t0 + i] | (uint32_t(__popcll(base & T.zy[t0 + i])) << 31);
   __syncthreads();
   const uint32_t even = uint32_t(S.ge - S.g0), odd = uint32_t(S.go - S.g0);
-  double acc = pauli_singles<false>(A, sh, 0, even, 0.0);
+  double acc = pauli_singles<false>(A, sh, 0, even, 0.0), diagonal = 0.0;
   acc = pauli_singles<true>(A, sh, even, odd, acc);
   for (uint32_t g = odd; g < uint32_t(S.g1 - S.g0); ++g) {
     const PauliTileGroup G = sh.group[g];
@@ -274,10 +274,10 @@ __device__ __forceinline__ double pauli_tile(const typename Vec2<Real>::T *__res
     else if (G.c)
       acc += pauli_group_any(sh, G, m);
     else if (FULL || rows)
-      acc += pauli_diagonal(sh, G, T.diag);
+      diagonal += pauli_diagonal(sh, G, T.diag);
   }
   __syncthreads();
-  return acc;
+  return fma(2.0, acc, diagonal);  // pairs count twice (not in the weights: those may be near the range's end)
 }
 
 // The carried sum partial[blockIdx.x], partial[gridDim.x + blockIdx.x] (+)=

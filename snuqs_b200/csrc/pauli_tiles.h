@@ -203,8 +203,8 @@ uint32_t plan_pauli_tiles(PauliTilePlan &P, uint32_t n, const Index *idx, uint32
       auto put = [&](uint32_t t, uint32_t zt) {
         P.zy[nt] = zym[t];
         // (-i)^ny folded into a real factor: even ny (-1)^(ny/2), odd ny
-        // (-1)^((ny-1)/2) for the imaginary part; a pair counts twice.
-        P.f[nt] = w[t] * (((ny[t] / 2) & 1) ? -1.0 : 1.0) * (x ? 2.0 : 1.0);
+        // (-1)^((ny-1)/2) for the imaginary part.
+        P.f[nt] = w[t] * (((ny[t] / 2) & 1) ? -1.0 : 1.0);
         P.zt[nt++] = zt;
       };
       auto coordinates = [&](uint32_t t) {

@@ -42,3 +42,20 @@ def test_ring_sum_rounding(n):
         st.close()
     rms = float(np.sqrt(np.mean(np.square(errors))))
     assert rms <= 4.0 * 2.0 ** -53 * n * 2.0 ** (-n / 2), rms
+
+
+@pytest.mark.parametrize("string", ["XXXXXXXXXXXX", "IIIIIIIIIIIX", "ZIIIIIIIIIII", "XIIIIIIIIIIY"])
+def test_weight_near_the_range_end(string):
+    """A finite weight times an expectation of at most 1 is finite: <P> = 1 on
+    the +1 eigenstate of the string's letters, every other product smaller."""
+    n, w = 12, 1.5e308
+    eig = {"I": [1, 0], "X": [1, 1], "Y": [1, 1j], "Z": [1, 0]}
+    psi = np.ones(1, dtype=np.complex128)
+    for c in string:
+        v = np.array(eig[c], dtype=np.complex128)
+        psi = np.kron(psi, v / np.linalg.norm(v))
+    st = capi.State(n, capi.SQ_C128)
+    st.from_host(psi)
+    got = st.expectation([(w, string)])
+    st.close()
+    assert np.isfinite(got) and abs(got - w) <= 1e-13 * w, got
