@@ -148,10 +148,11 @@ extern "C" int sq_expect_pauli_noalloc(const void *state, uint32_t num_qubits, i
   if (groups > sq::kPauliMaxGroups)
     return fail(SQ_ERR_UNSUPPORTED,
                 "sq_expect_pauli_noalloc: more than 256 distinct Pauli groups");
-  const uint32_t blocks = std::min(uint32_t(sms) * 4, kNoAllocMaxBlocks);
+  uint32_t blocks = std::min(uint32_t(sms) * 4, kNoAllocMaxBlocks);
   sq::PauliTilePlan P;  // 26 KiB on the stack
   if (sq::plan_pauli_tiles(P, n, idx, n_terms, 0, xm, zym, ny, weights, blocks) != n_terms)
     return fail(SQ_ERR_UNSUPPORTED, "sq_expect_pauli_noalloc: the terms do not fit one plan");
+  blocks = sq::pauli_tile_blocks(P, blocks);
   auto s = static_cast<cudaStream_t>(stream);
   // accumulate = 0: every used partial slot is overwritten, so the previous
   // call's contents need no clearing.
@@ -159,7 +160,7 @@ extern "C" int sq_expect_pauli_noalloc(const void *state, uint32_t num_qubits, i
                       : sq::launch_pauli_tiles<double>(state, P, partials, blocks, 0, s);
   if (e != cudaSuccess) return fail(SQ_ERR_CUDA, cudaGetErrorString(e));
   // Fixed-order sum of the partials into the caller's output (deterministic).
-  sq::finalize_carried_kernel<<<1, sq::kReduceThreads, 0, s>>>(partials, blocks, out_device);
+  sq::finalize_carried_kernel<<<1, sq::kReduceThreads, 0, s>>>(partials, blocks, out_device, nullptr);
   e = cudaGetLastError();
   if (e != cudaSuccess) return fail(SQ_ERR_CUDA, cudaGetErrorString(e));
   return SQ_OK;

@@ -75,13 +75,18 @@ __device__ __forceinline__ CarriedSum block_sum(CarriedSum v) {
   return v;
 }
 
-// out[0] = sum of the n carried sums partial[i], partial[n + i], in a fixed order.
+// out[0] = sum of the n carried sums partial[i], partial[n + i], in a fixed
+// order; out[1] takes *word (if any), for one copy to the host instead of two.
 static __global__ void __launch_bounds__(kReduceThreads)
-    finalize_carried_kernel(const double *__restrict__ partial, uint32_t n, double *__restrict__ out) {
+    finalize_carried_kernel(const double *__restrict__ partial, uint32_t n, double *__restrict__ out,
+                            const uint32_t *__restrict__ word) {
   CarriedSum v{0.0, 0.0};
   for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) carry_add(v, partial[i], partial[n + i]);
   v = block_sum(v);
-  if (threadIdx.x == 0) out[0] = carried(v);
+  if (threadIdx.x == 0) {
+    out[0] = carried(v);
+    if (word) *reinterpret_cast<uint32_t *>(out + 1) = *word;
+  }
 }
 
 __device__ __forceinline__ double pauli_signed(double v, uint32_t bit31) {
@@ -208,7 +213,8 @@ __device__ __forceinline__ double pauli_diagonal(const PauliShared &S, const Pau
 
 // Copies a pass's groups and terms to shared memory (term numbers from 0).
 // Ends without a barrier.
-__device__ __forceinline__ void pauli_stage(const PauliTilePlan &T, const PauliTilePass &S, PauliShared &sh) {
+template <class Plan>
+__device__ __forceinline__ void pauli_stage(const Plan &T, const PauliTilePass &S, PauliShared &sh) {
   const uint32_t t0 = T.group[S.g0].t0, t1 = T.group[S.g1 - 1].t1;
   const uint32_t singles = uint32_t(S.go - S.g0);  // their terms come first
   for (uint32_t i = threadIdx.x; i < t1 - t0; i += kPauliThreads) {
@@ -227,8 +233,8 @@ __device__ __forceinline__ void pauli_stage(const PauliTilePlan &T, const PauliT
 
 // Thread's share of all groups of one pass on tile `t`.  The pass is staged
 // in sh (its barrier is the one below); ends with a barrier.
-template <typename Real, bool FULL>
-__device__ __forceinline__ double pauli_tile(const typename Vec2<Real>::T *__restrict__ psi, const PauliTilePlan &T,
+template <typename Real, bool FULL, class Plan>
+__device__ __forceinline__ double pauli_tile(const typename Vec2<Real>::T *__restrict__ psi, const Plan &T,
                                              const PauliTilePass &S, uint64_t t, PauliShared &sh) {
   const uint32_t tid = threadIdx.x, low = T.low, m = T.m;
   uint64_t base = t << low;
@@ -282,23 +288,23 @@ __device__ __forceinline__ double pauli_tile(const typename Vec2<Real>::T *__res
 
 // The carried sum partial[blockIdx.x], partial[gridDim.x + blockIdx.x] (+)=
 // this block's share of the plan's expectation.
-template <typename Real, bool FULL>
+template <typename Real, bool FULL, class Plan>
 __global__ void __launch_bounds__(kPauliThreads, 4)
-    pauli_expect_tiles(const typename Vec2<Real>::T *__restrict__ psi, const __grid_constant__ PauliTilePlan T,
+    pauli_expect_tiles(const typename Vec2<Real>::T *__restrict__ psi, const __grid_constant__ Plan T,
                        double *__restrict__ partial, int accumulate) {
   extern __shared__ __align__(16) unsigned char pauli_raw[];
   PauliShared sh(pauli_raw, T.max_terms);
   const uint32_t tile_bits = T.n - T.m;
   const uint64_t items = uint64_t(T.npasses) << tile_bits;
   uint32_t staged = ~0u;
-  CarriedSum acc{0.0, 0.0};
+  double acc = 0.0;  // a thread's tiles alternate over the state: its sum stays small
   for (uint64_t w = blockIdx.x; w < items; w += gridDim.x) {
     const uint32_t pass = uint32_t(w >> tile_bits);
     if (pass != staged) pauli_stage(T, T.pass[pass], sh);
     staged = pass;
-    carry_add(acc, pauli_tile<Real, FULL>(psi, T, T.pass[pass], w & ((uint64_t(1) << tile_bits) - 1), sh), 0.0);
+    acc += pauli_tile<Real, FULL>(psi, T, T.pass[pass], w & ((uint64_t(1) << tile_bits) - 1), sh);
   }
-  CarriedSum s = block_sum(acc);
+  CarriedSum s = block_sum(CarriedSum{acc, 0.0});
   if (threadIdx.x == 0) {
     double *hi = partial + blockIdx.x, *lo = hi + gridDim.x;
     if (accumulate) carry_add(s, *hi, *lo);
@@ -307,12 +313,12 @@ __global__ void __launch_bounds__(kPauliThreads, 4)
   }
 }
 
-// Launches pauli_expect_tiles on `st` (2 x blocks partials).
-template <typename Real>
-inline cudaError_t launch_pauli_tiles(const void *psi, const PauliTilePlan &P, double *partial, uint32_t blocks,
-                                      int accumulate, cudaStream_t st) {
+// Launches the kernel of a plan on `st` (2 x blocks partials).
+template <typename Real, class Plan>
+inline cudaError_t launch_pauli_plan(const void *psi, const Plan &P, double *partial, uint32_t blocks, int accumulate,
+                                     cudaStream_t st) {
   const uint32_t smem = pauli_tile_smem(P.max_terms, P.max_groups);
-  auto fn = P.m == kPauliTileBits ? pauli_expect_tiles<Real, true> : pauli_expect_tiles<Real, false>;
+  auto fn = P.m == kPauliTileBits ? pauli_expect_tiles<Real, true, Plan> : pauli_expect_tiles<Real, false, Plan>;
   if (smem > 48 * 1024) {
     const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                int(pauli_tile_smem(kPauliMaxTerms, kPauliMaxGroups)));
@@ -320,6 +326,14 @@ inline cudaError_t launch_pauli_tiles(const void *psi, const PauliTilePlan &P, d
   }
   fn<<<blocks, kPauliThreads, smem, st>>>(static_cast<const typename Vec2<Real>::T *>(psi), P, partial, accumulate);
   return cudaGetLastError();
+}
+
+template <typename Real>
+inline cudaError_t launch_pauli_tiles(const void *psi, const PauliTilePlan &P, double *partial, uint32_t blocks,
+                                      int accumulate, cudaStream_t st) {
+  PauliSmallPlan S;
+  return pauli_small_plan(P, S) ? launch_pauli_plan<Real>(psi, S, partial, blocks, accumulate, st)
+                                : launch_pauli_plan<Real>(psi, P, partial, blocks, accumulate, st);
 }
 
 }  // namespace sq

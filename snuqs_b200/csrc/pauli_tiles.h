@@ -46,25 +46,58 @@ struct PauliTilePass {
 
 // Tile index j stands for global index base ^ (j's low bits) ^ gens of its
 // other bits; base runs over the indices with the low and pivot bits clear.
-struct PauliTilePlan {
+template <uint32_t TERMS, uint32_t GROUPS, uint32_t PASSES>
+struct PauliPlanOf {
   uint32_t n;
   uint32_t m, low;   // tile bits, low bits (both at most n)
   uint32_t npasses;
   uint32_t max_terms, max_groups;  // of any pass (shared-memory sizes)
-  PauliTilePass pass[kPauliMaxPasses];
-  PauliTileGroup group[kPauliMaxGroups];
-  uint64_t zy[kPauliMaxTerms];   // Z-or-Y mask (global index bits)
-  double f[kPauliMaxTerms];      // weight and phase
-  uint32_t zt[kPauliMaxTerms];   // Z-or-Y mask in tile coordinates
+  PauliTilePass pass[PASSES];
+  PauliTileGroup group[GROUPS];
+  uint64_t zy[TERMS];   // Z-or-Y mask (global index bits)
+  double f[TERMS];      // weight and phase
+  uint32_t zt[TERMS];   // Z-or-Y mask in tile coordinates
   // Terms of the diagonal group (at most one), relative to its first: those
   // with row parities z (tile bits 8..10 of zt) are diag[z] .. diag[z + 1].
   uint16_t diag[9];
 };
+using PauliTilePlan = PauliPlanOf<kPauliMaxTerms, kPauliMaxGroups, kPauliMaxPasses>;
+// A plan is a kernel argument: one of 26 KiB makes a call on a small state
+// longer than its two kernels (a norm of 2 qubits 53 us, with this one of
+// 3.4 KiB, which sums of up to some sixty strings fit, 41 us).
+using PauliSmallPlan = PauliPlanOf<96, 64, 12>;
+
+// Copies a plan to the small form; false when it does not fit.
+inline bool pauli_small_plan(const PauliTilePlan &P, PauliSmallPlan &S) {
+  const uint32_t groups = P.npasses ? P.pass[P.npasses - 1].g1 : 0, terms = groups ? P.group[groups - 1].t1 : 0;
+  if (P.npasses > 12 || groups > 64 || terms > 96) return false;
+  S.n = P.n;
+  S.m = P.m;
+  S.low = P.low;
+  S.npasses = P.npasses;
+  S.max_terms = P.max_terms;
+  S.max_groups = P.max_groups;
+  for (uint32_t i = 0; i < P.npasses; ++i) S.pass[i] = P.pass[i];
+  for (uint32_t i = 0; i < groups; ++i) S.group[i] = P.group[i];
+  for (uint32_t i = 0; i < terms; ++i) {
+    S.zy[i] = P.zy[i];
+    S.f[i] = P.f[i];
+    S.zt[i] = P.zt[i];
+  }
+  for (uint32_t i = 0; i < 9; ++i) S.diag[i] = P.diag[i];
+  return true;
+}
 
 // Dynamic shared memory of the kernels for passes of at most these sizes:
 // the tile as complex doubles, two 16-byte records per term, the groups.
 constexpr uint32_t pauli_tile_smem(uint32_t terms, uint32_t groups) {
   return (16u << kPauliTileBits) + groups * 8u + terms * 32u;
+}
+
+// Blocks of one launch: `most`, or as many as there are tiles to work.
+inline uint32_t pauli_tile_blocks(const PauliTilePlan &P, uint32_t most) {
+  const uint64_t items = uint64_t(P.npasses) << (P.n - P.m);
+  return items < 1 ? 1 : items < most ? uint32_t(items) : most;
 }
 
 // Plans the groups that start at term position `pos` of the term order idx
@@ -84,19 +117,22 @@ uint32_t plan_pauli_tiles(PauliTilePlan &P, uint32_t n, const Index *idx, uint32
   P.npasses = P.max_terms = P.max_groups = 0;
   // Groups [first, last) of the term order.
   uint16_t first[kPauliMaxGroups], last[kPauliMaxGroups];
-  bool taken[kPauliMaxGroups];
+  uint16_t open[kPauliMaxGroups];  // groups not yet in a pass
+  uint64_t mask[kPauliMaxGroups];  // flip masks without the low bits
   uint32_t ngroups = 0;
   const uint32_t base = pos;
+  const uint64_t lowmask = (uint64_t(1) << P.low) - 1;
   while (pos < nterms && ngroups < kPauliMaxGroups) {
     uint32_t end = pos;
     while (end < nterms && xm[idx[end]] == xm[idx[pos]] && (ny[idx[end]] & 1) == (ny[idx[pos]] & 1)) ++end;
     if (end - base > kPauliMaxTerms) break;
     first[ngroups] = uint16_t(pos - base);
     last[ngroups] = uint16_t(end - base);
-    taken[ngroups++] = false;
+    mask[ngroups] = xm[idx[pos]] & ~lowmask;
+    open[ngroups] = uint16_t(ngroups);
+    ++ngroups;
     pos = end;
   }
-  const uint64_t lowmask = (uint64_t(1) << P.low) - 1;
   const uint32_t gens = P.m - P.low;
   const uint64_t tiles = uint64_t(1) << (n - P.m);
   // Groups per pass: all that fit when the tiles alone fill the GPU.
@@ -110,38 +146,38 @@ uint32_t plan_pauli_tiles(PauliTilePlan &P, uint32_t n, const Index *idx, uint32
   for (uint32_t left = ngroups; left;) {
     if (P.npasses == kPauliMaxPasses) return base;  // cannot happen: see kPauliMaxPasses
     PauliTilePass &S = P.pass[P.npasses++];
-    uint64_t gen[kPauliGens];
-    uint32_t piv[kPauliGens], dim = 0;
+    uint64_t gen[kPauliGens] = {};
+    uint32_t piv[kPauliGens] = {}, dim = 0;
     bool val[kPauliGens];  // l(gen[i])
-    // gen stays reduced: bit piv[i] is set in gen[i] only.  Adds x with l(x) = v.
+    // gen stays reduced: bit piv[i] is set in gen[i] only, so the part of x
+    // outside the span follows from x's own pivot bits (every open group is
+    // tried in every pass: without branches 300 random strings on 17 qubits are
+    // planned in 54 us, with them in 170 us).  Adds x with l(x) = v.
     auto add = [&](uint64_t x, bool v) -> bool {
-      for (uint32_t i = 0; i < dim; ++i)
-        if ((x >> piv[i]) & 1) {
-          x ^= gen[i];
-          v ^= val[i];
-        }
-      if (!x) return true;
+      uint64_t rest = x;
+      for (uint32_t i = 0; i < kPauliGens; ++i) rest ^= gen[i] & (0 - ((x >> piv[i]) & 1));
+      if (!rest) return true;
       if (dim == gens) return false;
-      uint32_t p = 0;
-      while (!((x >> p) & 1)) ++p;
+      for (uint32_t i = 0; i < dim; ++i) v ^= val[i] & bool((x >> piv[i]) & 1);
+      const uint32_t p = uint32_t(__builtin_ctzll(rest));
       for (uint32_t i = 0; i < dim; ++i)
         if ((gen[i] >> p) & 1) {
-          gen[i] ^= x;
+          gen[i] ^= rest;
           val[i] ^= v;
         }
-      gen[dim] = x;
+      gen[dim] = rest;
       val[dim] = v;
       piv[dim++] = p;
       return true;
     };
     uint16_t member[kPauliMaxGroups];
-    uint32_t nm = 0;
-    for (uint32_t g = 0; g < ngroups && nm < cap; ++g)
-      if (!taken[g] && add(xm[idx[base + first[g]]] & ~lowmask, true)) {
-        taken[g] = true;
-        member[nm++] = uint16_t(g);
-      }
-    left -= nm;
+    uint32_t nm = 0, kept = 0;
+    for (uint32_t k = 0; k < left; ++k) {
+      const uint16_t g = open[k];
+      if (nm < cap && add(mask[g], true)) member[nm++] = g;
+      else open[kept++] = g;
+    }
+    left = kept;
     for (uint32_t b = P.low; dim < gens; ++b) add(uint64_t(1) << b, false);  // fill with the lowest free bits
     // The top tile bit: a generator with l = 1, which the others with l = 1
     // then lose; the rest in ascending pivot order.
