@@ -2,6 +2,7 @@
 import numpy as np
 import pytest
 
+import oracle
 from snuqs_b200 import capi
 
 pytestmark = pytest.mark.gpu
@@ -59,3 +60,23 @@ def test_weight_near_the_range_end(string):
     got = st.expectation([(w, string)])
     st.close()
     assert np.isfinite(got) and abs(got - w) <= 1e-13 * w, got
+
+
+@pytest.mark.parametrize("dtype", [capi.SQ_C128, capi.SQ_C64])
+@pytest.mark.parametrize("n", [10, 11, 12, 13, 16, 21])
+def test_flips_of_the_last_qubits(n, dtype):
+    """Strings of one flip within the last three qubits, alone (their own
+    kernel from a tile's size up), with several signs, and with others."""
+    rng = np.random.default_rng(n)
+    psi = rng.standard_normal(1 << n) + 1j * rng.standard_normal(1 << n)
+    psi = (psi / np.linalg.norm(psi)).astype(np.complex64 if dtype == capi.SQ_C64 else np.complex128)
+    st = capi.State(n, dtype)
+    st.from_host(psi)
+    for tail in ("IIX", "IIY", "IXI", "XIY", "YXX", "YYZ", "ZIX", "XXI"):
+        heads = ["".join(rng.choice(list("IZ"), n - 3)) for _ in range(3)]
+        one = [(float(rng.standard_normal()), h + tail) for h in heads]
+        other = [(0.7, "X" + "I" * (n - 1)), (-0.3, "I" * (n - 2) + "XX"), (0.2, "Z" * n)]
+        for terms in (one[:1], one, one + other):
+            got, want = st.expectation(terms), oracle.expectation_indexed(psi, n, terms)
+            assert abs(got - want) <= 1e-13 * sum(abs(w) for w, _ in terms), (tail, got, want)
+    st.close()
