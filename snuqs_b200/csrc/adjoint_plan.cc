@@ -77,7 +77,7 @@ void build_adjoint(const sq_circuit_op *ops, uint32_t nops, uint32_t n, AdjointP
     HostOp h;
     if (analyse_op(m, index_bits(op, n), 0, 0, h)) out.forward.push_back(h);
   }
-  std::map<std::pair<int32_t, double>, uint32_t> slot_of;
+  std::map<std::pair<int32_t, uint64_t>, uint32_t> slot_of;  // (parameter, bits of the factor)
   for (uint32_t i = nops; i-- > 0;) {
     const sq_circuit_op &op = ops[i];
     const int d = 1 << op.k;
@@ -106,9 +106,12 @@ void build_adjoint(const sq_circuit_op *ops, uint32_t nops, uint32_t n, AdjointP
           ip.m = K;
         }
         // Angles that follow one parameter with one factor share a slot.
-        const auto key = std::make_pair(int32_t(op.param[a]), double(op.scale[a]));
-        const auto it = slot_of.emplace(key, uint32_t(out.occurrences.size()));
-        if (it.second) out.occurrences.push_back(key);
+        // Compared by their bits: a NaN is not less than any number, nor any
+        // number less than it, and would take another factor's slot.
+        uint64_t bits;
+        std::memcpy(&bits, &op.scale[a], sizeof(bits));
+        const auto it = slot_of.emplace(std::make_pair(int32_t(op.param[a]), bits), uint32_t(out.occurrences.size()));
+        if (it.second) out.occurrences.push_back({op.param[a], op.scale[a]});
         ip.slot = it.first->second;
         out.reverse.push_back(ip);
       }
