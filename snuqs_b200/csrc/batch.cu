@@ -987,11 +987,13 @@ bool plan_gradient_circuit(const Circ &c, uint32_t m, std::vector<unsigned char>
     ropt.reg_bits = sq::kAdjRegBits;
     ropt.max_dense_k = sq::kAdjRegBits;
     if (multi) {
-      // Multi-state sweeps: the tiles of the single-state passes.
+      // Multi-state sweeps: the tiles of the single-state passes.  Tiles are
+      // selected by the planner's size rule: below it selection saves the
+      // device nothing here and costs the host a tenth of the call (64 sets of
+      // 12 qubits 2.8 ms with it, 2.5 ms without; 64 of 16 qubits 7.6 and 6.7).
       ropt.tile_bits = uint32_t(sq::kAdjTileBitsC128[2]);
       fopt.tile_bits = batch_default_bits<Real>();
       fopt.low_bits = multi_low_bits<Real>(c.n);
-      fopt.select = ropt.select = multi_select();
     }
     const auto fplan = share ? share->plan(ap.forward, c.n, fopt) : sq::plan_sweeps(ap.forward, c.n, fopt);
     const auto rplan = share ? share->plan(ap.reverse, c.n, ropt) : sq::plan_sweeps(ap.reverse, c.n, ropt);
