@@ -382,9 +382,13 @@ std::pair<uint64_t, uint64_t> structure_key(const std::vector<unsigned char> &p,
                                             const std::vector<std::pair<size_t, size_t>> &holes, uint32_t n) {
   uint64_t a = 1469598103934665603ull ^ n, b = 0x9ae16a3b2f90404full + n;
   auto mix = [&](size_t from, size_t to) {
-    for (size_t i = from; i < to; ++i) {
-      a = (a ^ p[i]) * 1099511628211ull;
-      b = (b ^ p[i]) * 0x100000001b3ull + 0x9e3779b97f4a7c15ull;
+    for (size_t i = from; i < to; i += 8) {
+      uint64_t w = 0;
+      std::memcpy(&w, p.data() + i, std::min<size_t>(8, to - i));
+      a = (a ^ w) * 0x9ddfea08eb382d69ull;
+      a ^= a >> 32;
+      b = (b ^ w) * 0xc2b2ae3d27d4eb4full + 0x9e3779b97f4a7c15ull;
+      b ^= b >> 29;
     }
   };
   size_t pos = 0;
@@ -1052,10 +1056,27 @@ struct MultiGradient {
 };
 
 // Kernels of the sweeps of one circuit's packed gradient plan in their
-// multi-state forms; false when one cannot be had.
+// multi-state forms; false when one cannot be had.  Looked up by the device and
+// the plan's structure, which is all that they and the rest depend on: hashing
+// and configuring the kernels sweep by sweep again took a third of the call for
+// four sets of 12 qubits.
 template <typename Real>
-bool multi_gradient_kernels(const std::vector<unsigned char> &plan, uint32_t nfwd, MultiGradient &G) {
+bool multi_gradient_kernels(int device, const std::vector<unsigned char> &plan, uint32_t n, uint32_t nfwd,
+                            uint32_t nrev, MultiGradient &G) {
   constexpr bool c64 = sizeof(Real) == 4;
+  constexpr size_t kMaxMemo = 256;
+  static std::mutex memo_mu;
+  static std::map<std::tuple<uint64_t, uint64_t, uint64_t, int>, MultiGradient> memo;
+  const auto sk = structure_key(plan, coef_ranges<Real>(plan), n);
+  const std::tuple<uint64_t, uint64_t, uint64_t, int> key{sk.first, sk.second, (uint64_t(nfwd) << 32) | nrev, device};
+  {
+    std::lock_guard<std::mutex> lk(memo_mu);
+    const auto it = memo.find(key);
+    if (it != memo.end()) {
+      G = it->second;
+      return true;
+    }
+  }
   std::vector<uint64_t> coef_at;
   const std::vector<sq::PlannedSweep> sweeps = unpack_sweeps(plan, coef_at);
   const uint32_t MF = batch_default_bits<Real>();
@@ -1100,6 +1121,24 @@ bool multi_gradient_kernels(const std::vector<unsigned char> &plan, uint32_t nfw
       G.tile_bits.push_back(ps.h.m);
     }
   }
+  std::lock_guard<std::mutex> lk(memo_mu);
+  if (memo.size() >= kMaxMemo) memo.clear();
+  memo[key] = G;
+  return true;
+}
+
+// What parameter sets of one program have in common: as many gates, on the same
+// qubits, following the same parameters, and the same angles zero (the value
+// that drops a gate or gives it another form).
+bool one_arrangement(const Circ &a, const Circ &b) {
+  if (a.n != b.n || a.ops.size() != b.ops.size()) return false;
+  for (size_t i = 0; i < a.ops.size(); ++i) {
+    const sq_circuit_op &x = a.ops[i], &y = b.ops[i];
+    if (x.k != y.k || x.nangles != y.nangles || !std::equal(x.qubits, x.qubits + std::min(x.k, 3u), y.qubits))
+      return false;
+    for (uint32_t j = 0; j < std::min(x.nangles, 3u); ++j)
+      if (x.param[j] != y.param[j] || (x.angles[j] == 0.0) != (y.angles[j] == 0.0)) return false;
+  }
   return true;
 }
 
@@ -1123,29 +1162,30 @@ int run_gradient_impl(sq_batch *b, uint32_t n_params, double *energies, double *
   std::vector<std::vector<std::pair<int32_t, double>>> occs(nc);
   std::vector<std::string> errs(nc);
   std::vector<char> ok(nc, 0);
-  std::atomic<size_t> next{0};
   const unsigned nth = std::max(1u, std::min(16u, std::thread::hardware_concurrency()));
-  // complex128 circuits of one size above the tile are planned for multi-state
-  // sweeps (parameter sets of one circuit); when their plans turn out to
-  // differ, for the kernel that runs one circuit per CTA.  complex64 stays
-  // with that kernel: the multi-state reverse sweeps take smaller tiles, and
-  // another plan is another order of FP32 roundings, which the FP64 gradients
-  // show.
+  // complex128 parameter sets of one program above the tile are planned for
+  // multi-state sweeps.  Circuits that differ are told apart before planning:
+  // when their plans turn out to differ they are planned again, for the kernel
+  // that runs one circuit per CTA (64 circuits of 14 qubits 10.8 ms planned
+  // twice, 7.2 ms once).  complex64 stays with that kernel: the multi-state
+  // reverse sweeps take smaller tiles, and another plan is another order of
+  // FP32 roundings, which the FP64 gradients show.
   bool try_multi = sizeof(Real) == 8 && multi_enabled() && b->circs[0].n > M && b->circs[0].n >= sq::kApplyBits;
-  for (size_t i = 1; i < nc; ++i) try_multi = try_multi && b->circs[i].n == b->circs[0].n;
+  for (size_t i = 1; i < nc && try_multi; ++i) try_multi = one_arrangement(b->circs[0], b->circs[i]);
   auto plan_all = [&](bool as_multi) {
     PlanShare share;
-    next = 0;
-    std::vector<std::thread> workers;
-    for (unsigned t = 0; t < nth; ++t)
-      workers.emplace_back([&]() {
-        for (size_t i = next++; i < nc; i = next++) {
-          packed[i].clear();
-          occs[i].clear();
-          ok[i] = plan_gradient_circuit<Real>(b->circs[i], M, packed[i], nfwd[i], nrev[i], occs[i], errs[i], &share,
-                                              as_multi);
-        }
-      });
+    std::atomic<size_t> next{0};
+    auto work = [&] {
+      for (size_t i = next++; i < nc; i = next++) {
+        packed[i].clear();
+        occs[i].clear();
+        ok[i] = plan_gradient_circuit<Real>(b->circs[i], M, packed[i], nfwd[i], nrev[i], occs[i], errs[i], &share,
+                                            as_multi);
+      }
+    };
+    std::vector<std::thread> workers;  // and this thread: none for one circuit
+    for (size_t t = 1; t < std::min<size_t>(nth, nc); ++t) workers.emplace_back(work);
+    work();
     for (auto &th : workers) th.join();
   };
   plan_all(try_multi);
@@ -1153,8 +1193,9 @@ int run_gradient_impl(sq_batch *b, uint32_t n_params, double *energies, double *
     bool fine = true;
     for (size_t i = 0; i < nc; ++i) fine = fine && ok[i];
     fine = fine && uniform_plans<Real>(b, packed, nfwd, nrev, occs, M) &&
-           multi_gradient_kernels<Real>(packed[0], nfwd[0], multi);
+           multi_gradient_kernels<Real>(b->device, packed[0], b->circs[0].n, nfwd[0], nrev[0], multi);
     if (!fine) {
+      multi = MultiGradient();
       try_multi = false;
       plan_all(false);
     }
