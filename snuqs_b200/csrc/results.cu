@@ -14,7 +14,7 @@
 // amplitudes, then pairs of pairs, ...), and a shot with uniform u walks that
 // tree from the root with r = u * total: at a node with children sums (L, R)
 // it goes left when r < L or R == 0, else subtracts L and goes right.  The
-// tree is cut at nodes of 2^7 amplitudes: the levels from there up stay in
+// tree is cut at nodes of 2^7 (2^5) amplitudes: the levels from there up stay in
 // device memory, the levels inside a node are rebuilt in registers by the warp
 // that serves a shot.  Any restatement that sums in the same tree and walks
 // it the same way returns the same indices.
@@ -37,15 +37,22 @@ namespace {
 
 // Amplitudes of one block of the first pass, and the size of the nodes that
 // the stored tree ends at: 2^7 amplitudes up to 30 qubits, then as large as
-// keeps the stored tree at 2^24 doubles (128 MiB).
+// keeps the stored tree at 2^24 doubles (128 MiB).  Nodes of 2^5 where the
+// shots together would read more than the state in nodes of 2^7 and the two
+// further levels are small (at most 16 MiB, up to 25 qubits): 10^6 shots of 20 /
+// 23 qubits complex128 195 / 231 us on the device, with nodes of 2^7 396 / 428 us
+// (with leaves of 2^12 summed again by blocks 509 / 204 us).
 constexpr int kBlockBits = 12;
 constexpr uint32_t kBlockAmps = 1u << kBlockBits;
 constexpr int kTreeThreads = 256;
 constexpr uint32_t kPerLane = kBlockAmps / kTreeThreads;  // 16 amplitudes, 32 apart
-constexpr uint32_t kNodeBits = 7;
+constexpr uint32_t kNodeBits = 7, kFineBits = 5;
 constexpr uint32_t kMaxTreeDepth = 23;
 
-uint32_t node_bits(uint32_t n) { return n > kNodeBits + kMaxTreeDepth ? n - kMaxTreeDepth : kNodeBits; }
+uint32_t node_bits(uint32_t n, uint64_t shots) {
+  if (n <= 25 && shots >= (uint64_t(1) << n) >> kNodeBits) return kFineBits;
+  return n > kNodeBits + kMaxTreeDepth ? n - kMaxTreeDepth : kNodeBits;
+}
 
 template <typename C2>
 __device__ __forceinline__ double prob_of(const C2 &a) {
@@ -85,11 +92,15 @@ __global__ void __launch_bounds__(kTreeThreads) node_sum_kernel(const C2 *__rest
   for (int o = 1; o < 32; o <<= 1)
 #pragma unroll
     for (uint32_t k = 0; k < kPerLane; ++k) v[k] = __dadd_rn(v[k], __shfl_xor_sync(0xffffffffu, v[k], o));
+  if (node <= kFineBits && lane == 0) {
+#pragma unroll
+    for (uint32_t j = 0; j < kPerLane; ++j) put(kFineBits, warp * kPerLane + j, v[j]);
+  }
 #pragma unroll
   for (uint32_t w = kPerLane / 2, s = 6; w >= 1; w >>= 1, ++s) {
 #pragma unroll
     for (uint32_t j = 0; j < w; ++j) v[j] = __dadd_rn(v[2 * j], v[2 * j + 1]);
-    if (s >= kNodeBits && s >= node && lane == 0) {
+    if (s >= node && lane == 0) {
 #pragma unroll
       for (uint32_t j = 0; j < w; ++j) put(s, warp * w + j, v[j]);
     }
@@ -156,7 +167,8 @@ __device__ __forceinline__ void prob4(const C2 *__restrict__ psi, uint64_t i, ui
 // 4l..4l+3 of the shot's 128-amplitude node, the five levels above them are
 // lane pairs as in node_sum_kernel, and the walk goes on in registers.
 // EXTRA > 0 (more than 30 qubits): the stored nodes hold 2^EXTRA runs of 128
-// amplitudes, whose sums are rebuilt first.
+// amplitudes, whose sums are rebuilt first.  EXTRA = -2: nodes of 32, one
+// amplitude a lane.
 // A shot reads 128 amplitudes, wherever it falls; before, each leaf of 2^12
 // amplitudes that any shot fell into was read and summed again by a block, for
 // many shots the whole state a second time, after a counting sort of the
@@ -218,11 +230,17 @@ __global__ void __launch_bounds__(256) shot_kernel(const C2 *__restrict__ psi, u
       }
       base += uint64_t(at - B) * 128;
     }
-    prob4(psi, base + 4 * lane, N, p);
-    const double lo = __dadd_rn(p[0], p[1]), hi = __dadd_rn(p[2], p[3]);
+    constexpr uint32_t PER = EXTRA < 0 ? 1 : 4;
+    if constexpr (EXTRA < 0) p[0] = base + lane < N ? prob_of(psi[base + lane]) : 0.0;
+    else prob4(psi, base + 4 * lane, N, p);
+    double lo = p[0], hi = 0.0;
+    if constexpr (EXTRA >= 0) {
+      lo = __dadd_rn(p[0], p[1]);
+      hi = __dadd_rn(p[2], p[3]);
+    }
     // sum[e]: the run of 2^e lanes this lane belongs to.
     double sum[5];
-    sum[0] = __dadd_rn(lo, hi);
+    sum[0] = EXTRA < 0 ? lo : __dadd_rn(lo, hi);
 #pragma unroll
     for (int e = 0; e < 4; ++e) sum[e + 1] = __dadd_rn(sum[e], __shfl_xor_sync(kAll, sum[e], 1 << e));
     uint32_t at = 0;  // first lane of the node walked to
@@ -236,15 +254,17 @@ __global__ void __launch_bounds__(256) shot_kernel(const C2 *__restrict__ psi, u
     }
     if (lane == at) {
       uint32_t a = 0;
-      double l = p[0], q = p[1];
-      if (!go_left(rr, lo, hi)) {
-        rr = __dsub_rn(rr, lo);
-        a = 2;
-        l = p[2];
-        q = p[3];
+      if constexpr (EXTRA >= 0) {
+        double l = p[0], q = p[1];
+        if (!go_left(rr, lo, hi)) {
+          rr = __dsub_rn(rr, lo);
+          a = 2;
+          l = p[2];
+          q = p[3];
+        }
+        if (!go_left(rr, l, q)) ++a;
       }
-      if (!go_left(rr, l, q)) ++a;
-      out[first + j] = base + 4 * lane + a;
+      out[first + j] = base + PER * lane + a;
     }
   }
 }
@@ -464,8 +484,8 @@ int fail(int code, const std::string &msg) { return sq_detail_fail(code, msg.c_s
 size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 
 // Scratch bytes of sample_impl: the stored tree.
-size_t sample_scratch_bytes(uint32_t n) {
-  const uint32_t node = node_bits(n);
+size_t sample_scratch_bytes(uint32_t n, uint64_t shots) {
+  const uint32_t node = node_bits(n, shots);
   return align256((uint64_t(2) << (n > node ? n - node : 0)) * sizeof(double));
 }
 
@@ -476,7 +496,7 @@ template <typename C2>
 int sample_impl(const C2 *psi, uint32_t n, const double *u, uint64_t shots, uint64_t *out, void *scr,
                 cudaStream_t st, cudaEvent_t u_ready = nullptr, const std::function<int()> &before_shots = {}) {
   double *tree = static_cast<double *>(scr);
-  const uint32_t node = node_bits(n);
+  const uint32_t node = node_bits(n, shots);
   const uint32_t blocks_log = n > uint32_t(kBlockBits) ? n - kBlockBits : 0;
   node_sum_kernel<C2><<<1u << blocks_log, kTreeThreads, 0, st>>>(psi, n, node, tree);
   RQ_CUDA(cudaGetLastError());
@@ -497,7 +517,8 @@ int sample_impl(const C2 *psi, uint32_t n, const double *u, uint64_t shots, uint
   while (per_warp > 1 && shots / per_warp < 148 * 64) per_warp >>= 1;
   const uint64_t warps = (shots + per_warp - 1) / per_warp;
   const unsigned grid = unsigned((warps + 7) / 8);
-  switch (node - kNodeBits) {
+  switch (int(node) - int(kNodeBits)) {
+    case -2: shot_kernel<C2, -2><<<grid, 256, 0, st>>>(psi, n, tree, u, shots, per_warp, out); break;
     case 0: shot_kernel<C2, 0><<<grid, 256, 0, st>>>(psi, n, tree, u, shots, per_warp, out); break;
     case 1: shot_kernel<C2, 1><<<grid, 256, 0, st>>>(psi, n, tree, u, shots, per_warp, out); break;
     case 2: shot_kernel<C2, 2><<<grid, 256, 0, st>>>(psi, n, tree, u, shots, per_warp, out); break;
@@ -521,7 +542,7 @@ int sq_sample(sq_state *s, const double *uniforms_device, uint64_t shots, uint64
   const uint32_t n = sq_state_num_qubits(s);
   if (n > 34) return fail(SQ_ERR_UNSUPPORTED, "sq_sample: more than 34 qubits");
   void *scr = nullptr;
-  const int sc = sq_detail_state_scratch(s, sample_scratch_bytes(n), &scr);
+  const int sc = sq_detail_state_scratch(s, sample_scratch_bytes(n, shots), &scr);
   if (sc != SQ_OK) return sc;
   if (sq_state_dtype(s) == SQ_C64)
     return sample_impl(static_cast<const float2 *>(sq_state_data(s)), n, uniforms_device, shots, out_device, scr, st);
@@ -540,7 +561,7 @@ int sq_sample_host(sq_state *s, const double *uniforms, uint64_t shots, uint64_t
   // The state's scratch holds the uniforms and the indices, then the sampler's own scratch.
   const size_t b_u = align256(shots * sizeof(double)), b_o = align256(shots * sizeof(uint64_t));
   void *scr = nullptr;
-  rc = sq_detail_state_scratch(s, b_u + b_o + sample_scratch_bytes(n), &scr);
+  rc = sq_detail_state_scratch(s, b_u + b_o + sample_scratch_bytes(n, shots), &scr);
   if (rc != SQ_OK) return rc;
   char *p = static_cast<char *>(scr);
   double *du = reinterpret_cast<double *>(p);
