@@ -125,7 +125,7 @@ __global__ void __launch_bounds__(kTreeThreads) node_sum_kernel(const C2 *__rest
 // from node b << levels, through shared memory.
 constexpr uint32_t kUpperLevels = 11;
 __global__ void __launch_bounds__(1024) upper_tree_kernel(double *__restrict__ tree, uint32_t from, uint32_t levels) {
-  __shared__ double buf[2][1u << (kUpperLevels - 1)];
+  __shared__ __align__(16) double buf[2][1u << (kUpperLevels - 1)];  // read in pairs
   uint32_t nodes = 1u << levels;
   const double2 *src = reinterpret_cast<const double2 *>(tree + ((uint64_t(1) << from) + (uint64_t(blockIdx.x) << levels)));
   for (uint32_t l = 1; l <= levels; ++l) {
