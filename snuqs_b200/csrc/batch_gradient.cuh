@@ -15,7 +15,7 @@ constexpr uint32_t kApplyBits = 12;  // amplitudes of one block
 // lambda = H psi over K states of 2^n amplitudes that lie back to back (state c
 // with Hamiltonian circuits[c].ham); partials[block] receives the block's
 // share of Re <psi|lambda>, 2^(n - kApplyBits) blocks per state.  Bound: one read
-// of psi and one write of lambda per flip group.
+// of psi per flip group and one for the energy, and one write of lambda.
 template <typename Real>
 __global__ void __launch_bounds__(kReduceThreads)
     batch_apply_kernel(const typename Vec2<Real>::T *__restrict__ psi, typename Vec2<Real>::T *__restrict__ lam,

@@ -513,8 +513,11 @@ int sample_impl(const C2 *psi, uint32_t n, const double *u, uint64_t shots, uint
   if (u_ready) RQ_CUDA(cudaStreamWaitEvent(st, u_ready, 0));
   // Shots per warp: as many as leave a warp for every slot of the GPU, at most
   // 32 (a warp serves its shots one after the other).
+  int dev = 0, sms = 0;
+  RQ_CUDA(cudaGetDevice(&dev));
+  RQ_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   uint32_t per_warp = 32;
-  while (per_warp > 1 && shots / per_warp < 148 * 64) per_warp >>= 1;
+  while (per_warp > 1 && shots / per_warp < uint64_t(sms) * 64) per_warp >>= 1;
   const uint64_t warps = (shots + per_warp - 1) / per_warp;
   const unsigned grid = unsigned((warps + 7) / 8);
   switch (int(node) - int(kNodeBits)) {
