@@ -305,7 +305,7 @@ int sq_adjoint_gradient(sq_state *psi, sq_state *lam, const sq_circuit_op *ops,
  * streams, no ordering) race; order them.  Limits: n_terms <= 1024 and at
  * most 256 distinct (X/Y mask, Y parity) groups; larger requests return
  * SQ_ERR_UNSUPPORTED.  A call stages the grouped terms on the calling
- * thread's stack (about 50 KiB). */
+ * thread's stack (about 57 KiB). */
 int sq_expect_pauli_noalloc(const void *state, uint32_t num_qubits, int dtype,
                             const char *paulis, const double *weights,
                             uint32_t n_terms, double *out_device, void *stream);

@@ -23,7 +23,7 @@
 // (16 KiB of FP64 partials), at most 1024 Pauli terms and 256 distinct
 // (X/Y mask, Y parity) groups per call.  Larger requests are rejected.
 // Each call stages the grouped terms on the calling thread's stack (about
-// 50 KiB: the kernel's parameter block and four term arrays).
+// 57 KiB: the plan, the kernel's parameter block and four term arrays).
 #include <cuda_runtime.h>
 
 #include <algorithm>

@@ -39,7 +39,8 @@ namespace {
 // the stored tree ends at: 2^7 amplitudes up to 30 qubits, then as large as
 // keeps the stored tree at 2^24 doubles (128 MiB).  Nodes of 2^5 where the
 // shots together would read more than the state in nodes of 2^7 and the two
-// further levels are small (at most 16 MiB, up to 25 qubits): 10^6 shots of 20 /
+// further levels are small (at most 16 MiB, up to 25 qubits), from 2^14 shots
+// (below, a call is its launches and copies): 10^6 shots of 20 /
 // 23 qubits complex128 195 / 231 us on the device, with nodes of 2^7 396 / 428 us
 // (with leaves of 2^12 summed again by blocks 509 / 204 us).
 constexpr int kBlockBits = 12;
@@ -50,7 +51,7 @@ constexpr uint32_t kNodeBits = 7, kFineBits = 5;
 constexpr uint32_t kMaxTreeDepth = 23;
 
 uint32_t node_bits(uint32_t n, uint64_t shots) {
-  if (n <= 25 && shots >= (uint64_t(1) << n) >> kNodeBits) return kFineBits;
+  if (n <= 25 && shots >= std::max(uint64_t(1) << 14, (uint64_t(1) << n) >> kNodeBits)) return kFineBits;
   return n > kNodeBits + kMaxTreeDepth ? n - kMaxTreeDepth : kNodeBits;
 }
 

@@ -20,7 +20,7 @@ def test_node_sizes(n, dtype):
     psi = (psi / np.linalg.norm(psi)).astype(np.complex64 if dtype == capi.SQ_C64 else np.complex128)
     st = capi.State(n, dtype)
     st.from_host(psi)
-    rule = max(2, (1 << n) >> 7)
+    rule = max(1 << 14, (1 << n) >> 7)
     u = np.concatenate([[0.0, np.nextafter(1.0, 0.0)], rng.random(rule)])
     want = oracle.sample_inverse_cdf(psi, u)
     for shots in (1, rule - 1, rule, rule + 2):
